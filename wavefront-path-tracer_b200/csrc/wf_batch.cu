@@ -181,10 +181,9 @@ __global__ void __maxnreg__(72) k_batch_trace(BatchView b, PathSoA ps, const uin
     L.stage = kStageDone;
     const DeviceScene* sp = nullptr;
     uint32_t i = 0;
-    bool more = true;
-    for (;;) {
-        bool idle = L.stage == kStageDone;
-        uint32_t slot = refill(&c->work_trace, n, idle, refill_at, more);
+    RayFeed feed;
+    uint32_t slot = feed_begin(feed, n);
+    for (;; slot = feed_next(feed, &c->work_trace, L.stage == kStageDone, refill_at)) {
         if (slot != kInvalid) {
             i = slot;
             uint32_t p = queue[i];
@@ -198,7 +197,7 @@ __global__ void __maxnreg__(72) k_batch_trace(BatchView b, PathSoA ps, const uin
         }
         bool busy = L.stage != kStageDone;
         if (!__any_sync(0xffffffffu, busy)) {
-            if (!more) break;
+            if (!feed.more) break;
             continue;
         }
         if (busy) {
@@ -267,10 +266,9 @@ __global__ void k_batch_shadow(BatchView b, const float4* shadow_origin, const f
     L.stage = kStageDone;
     const DeviceScene* sp = nullptr;
     uint32_t j = 0;
-    bool more = true;
-    for (;;) {
-        bool idle = L.stage == kStageDone;
-        uint32_t slot = refill(&c->work_shadow, n, idle, refill_at, more);
+    RayFeed feed;
+    uint32_t slot = feed_begin(feed, n);
+    for (;; slot = feed_next(feed, &c->work_shadow, L.stage == kStageDone, refill_at)) {
         if (slot != kInvalid) {
             j = slot;
             float4 o = shadow_origin[j], d = shadow_dir[j];
@@ -280,7 +278,7 @@ __global__ void k_batch_shadow(BatchView b, const float4* shadow_origin, const f
         }
         bool busy = L.stage != kStageDone;
         if (!__any_sync(0xffffffffu, busy)) {
-            if (!more) break;
+            if (!feed.more) break;
             continue;
         }
         if (busy) {

@@ -164,10 +164,9 @@ WF_DEV void trace_stage(const DeviceScene& s, PathSoA ps, const uint32_t* queue,
     ClosestLane L;
     L.stage = kStageDone;
     uint32_t i = 0;
-    bool more = true;
-    for (;;) {
-        bool idle = L.stage == kStageDone;
-        uint32_t slot = refill(counter, n, idle, refill_at, more);
+    RayFeed feed;
+    uint32_t slot = feed_begin(feed, n);
+    for (;; slot = feed_next(feed, counter, L.stage == kStageDone, refill_at)) {
         if (slot != kInvalid) {
             i = first + slot;
             uint32_t p = queue[i];
@@ -180,7 +179,7 @@ WF_DEV void trace_stage(const DeviceScene& s, PathSoA ps, const uint32_t* queue,
         }
         bool busy = L.stage != kStageDone;
         if (!__any_sync(0xffffffffu, busy)) {
-            if (!more) break;
+            if (!feed.more) break;
             continue;
         }
         if (busy) {
@@ -405,10 +404,9 @@ WF_DEV void shadow_stage(DeviceScene s, const float4* shadow_origin, const float
     AnyLane L;
     L.stage = kStageDone;
     uint32_t j = 0;
-    bool more = true;
-    for (;;) {
-        bool idle = L.stage == kStageDone;
-        uint32_t slot = refill(&c->work_shadow, n, idle, refill_at, more);
+    RayFeed feed;
+    uint32_t slot = feed_begin(feed, n);
+    for (;; slot = feed_next(feed, &c->work_shadow, L.stage == kStageDone, refill_at)) {
         if (slot != kInvalid) {
             j = slot;
             float4 o = shadow_origin[j], d = shadow_dir[j];
@@ -417,7 +415,7 @@ WF_DEV void shadow_stage(DeviceScene s, const float4* shadow_origin, const float
         }
         bool busy = L.stage != kStageDone;
         if (!__any_sync(0xffffffffu, busy)) {
-            if (!more) break;
+            if (!feed.more) break;
             continue;
         }
         if (busy) {
