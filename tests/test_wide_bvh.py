@@ -1,0 +1,197 @@
+"""The compressed wide BVH against the BVH2s it is made from, on the CPU.
+
+A host build of the construction and traversal code (tests/wide_bvh_host.cpp)
+traces every ray twice, through the wide nodes and through the BVH2s, and the
+hits (distance, barycentrics, primitive, instance) and occlusion answers must
+agree bit for bit.  The rays are those where the two could part: axis-parallel
+ones with zero and denormal components, origins on box planes, through shared
+vertices and edges, grazing, from far away and from inside, with directions of
+other lengths than 1; the scenes flat, degenerate, duplicated, tiny, huge,
+scaled instances, and past the range the wide test covers."""
+import ctypes as C
+import shutil
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+from helpers import acceleration_cases, acceleration_rays
+from wfpt import abi, scenes
+from wfpt.native import Scene, material
+
+ROOT = Path(__file__).resolve().parents[1]
+CSRC = ROOT / "wavefront-path-tracer_b200" / "csrc"
+CUDA_INCLUDE = Path("/usr/local/cuda/include")
+
+
+@pytest.fixture(scope="module")
+def check(tmp_path_factory):
+    compiler = shutil.which("g++")
+    if compiler is None or not (CUDA_INCLUDE / "cuda_runtime.h").exists():
+        pytest.skip("needs g++ and the CUDA headers")
+    out = tmp_path_factory.mktemp("wide") / "libwide.so"
+    subprocess.run([compiler, "-O2", "-std=c++17", "-fPIC", "-shared", "-ffp-contract=off", "-pthread", "-w",
+                    f"-I{CSRC}", f"-I{CUDA_INCLUDE}", "-o", str(out), str(ROOT / "tests" / "wide_bvh_host.cpp"),
+                    str(CSRC / "wf_scene.cpp"), str(CSRC / "bvh_build.cpp")], check=True)
+    lib = C.CDLL(str(out))
+
+    def run(scene, rays, limits=None):
+        rays = np.ascontiguousarray(rays, abi.RAY_DTYPE)
+        if limits is None:
+            limits = np.random.default_rng(3).uniform(0.1, 20.0, len(rays))
+        limits = np.ascontiguousarray(limits, np.float32)
+        desc, keep = scene.desc()
+        counts = np.zeros(9, np.uint64)
+        status = lib.wide_check(C.byref(desc), C.c_void_p(rays.ctypes.data), C.c_void_p(limits.ctypes.data),
+                                C.c_uint32(len(rays)), C.c_void_p(counts.ctypes.data))
+        assert status == 0
+        names = ("closest", "any", "rays", "nodes", "wide_visits", "binary_visits", "usable", "redone", "hits")
+        got = dict(zip(names, (int(v) for v in counts)))
+        assert got["closest"] == 0 and got["any"] == 0, got
+        return got
+    return run
+
+
+def make_rays(origins, directions):
+    rays = np.zeros(len(origins), abi.RAY_DTYPE)
+    rays["origin"], rays["direction"] = origins, directions
+    return rays
+
+
+def hard_rays(points, extent, seed, count=6000):
+    """Rays among and at the given points (vertices of the scene): zero and
+    denormal components, origins on the points' planes, exact aims at them."""
+    rng = np.random.default_rng(seed)
+    p = points[rng.integers(0, len(points), count)].astype(np.float32)
+    o = rng.uniform(-1.5, 1.5, (count, 3)).astype(np.float32) * np.float32(extent)
+    d = rng.normal(0, 1, (count, 3)).astype(np.float32)
+    kind = rng.integers(0, 8, count)
+    aim = kind <= 2
+    d[aim] = p[aim] - o[aim]                                 # through a vertex, any length
+    on = kind == 3
+    axis = rng.integers(0, 3, count)
+    d[on] = 0.0
+    d[on, axis[on]] = np.where(rng.random(on.sum()) < 0.5, 1.0, -1.0)
+    o[on] = np.where(np.arange(3)[None] == axis[on][:, None], o[on], p[on])  # axis-parallel through a vertex
+    zero = kind == 4
+    d[zero, axis[zero]] = 0.0                                # in an axis plane, from a vertex's plane
+    o[zero, axis[zero]] = p[zero, axis[zero]]
+    tiny = kind == 5
+    d[tiny, axis[tiny]] = rng.choice([1e-40, -1e-40, 1e-30, -0.0, 1e-12], tiny.sum())
+    start = kind == 6
+    o[start] = p[start]                                      # from a vertex
+    d[np.abs(d).max(1) == 0] = (0, 0, 1)
+    return make_rays(o, d)
+
+
+def soup(n, seed, flat=False, size=0.2):
+    rng = np.random.default_rng(seed)
+    c = rng.uniform(-1, 1, (n, 1, 3))
+    v = (c + rng.normal(0, size, (n, 3, 3))).astype(np.float32)
+    if flat:
+        v[: n // 2, :, 1] = np.round(v[: n // 2, :1, 1] * 4) / 4   # axis-aligned triangles on few planes
+    v[::17, 2] = v[::17, 1]                                       # degenerate
+    v[1::13] = v[0]                                               # duplicates
+    return v
+
+
+def mesh_scene(v, *instances):
+    s = Scene()
+    m = s.add_material(material(abi.MAT_DIFFUSE, (0.5, 0.5, 0.5)))
+    s.add_mesh(scenes.triangles(v[:, 0], v[:, 1], v[:, 2], m))
+    s.instances = np.concatenate(instances) if instances else scenes.instance(0)
+    return s
+
+
+@pytest.mark.parametrize("name", list(acceleration_cases()))
+def test_acceleration_cases(check, name):
+    check(acceleration_cases()[name], acceleration_rays(count=4096))
+
+
+@pytest.mark.parametrize("count", [1, 2, 3, 4, 7, 8, 9, 24, 25, 200, 3000])
+@pytest.mark.parametrize("flat", [False, True])
+def test_triangle_soups(check, count, flat):
+    v = soup(count, count, flat)
+    got = check(mesh_scene(v), hard_rays(v.reshape(-1, 3), 1.0, count))
+    assert got["usable"] == 1
+
+
+def test_grid_of_shared_edges(check):
+    """A flat and a bumpy grid: rays at vertices and along edges meet several
+    triangles at one distance, which the BVH2s decide."""
+    n = 24
+    x, z = np.meshgrid(np.linspace(-1, 1, n + 1), np.linspace(-1, 1, n + 1), indexing="ij")
+    for bump in (0.0, 0.2):
+        p = np.stack([x, bump * np.sin(3 * x) * np.cos(2 * z), z], -1).astype(np.float32)
+        a, b, c, d = p[:-1, :-1], p[:-1, 1:], p[1:, 1:], p[1:, :-1]
+        v = np.concatenate([np.stack([a, b, c], 2).reshape(-1, 3, 3), np.stack([a, c, d], 2).reshape(-1, 3, 3)])
+        got = check(mesh_scene(v), hard_rays(v.reshape(-1, 3), 1.0, 5, 20000))
+        assert got["redone"] > 100
+
+
+@pytest.mark.parametrize("scale,offset", [(1e-9, 0.0), (1e-4, 0.0), (1e3, 0.0), (1.0, 3e4), (1e-3, 1e3), (1e6, 0.0)])
+def test_scales_and_offsets(check, scale, offset):
+    v = (soup(800, 4, flat=True).astype(np.float64) * scale + offset).astype(np.float32)
+    rays = hard_rays(soup(800, 4, flat=True).reshape(-1, 3), 1.0, 6)
+    rays["origin"] = rays["origin"] * np.float32(scale) + np.float32(offset)
+    got = check(mesh_scene(v), rays, np.random.default_rng(1).uniform(0, 3 * scale, len(rays)))
+    assert got["usable"] == 1 and (got["hits"] > 0 or scale < 1e-6)  # hits start at t = 1e-6
+
+
+@pytest.mark.parametrize("length", [1e-30, 1e-7, 1e-3, 1e3, 1e7, 1e30])
+def test_direction_lengths_and_far_origins(check, length):
+    v = soup(500, 8)
+    rays = hard_rays(v.reshape(-1, 3), 1.0, 9)
+    rays["direction"] *= np.float32(length)
+    check(mesh_scene(v), rays)
+    far = hard_rays(v.reshape(-1, 3), 1.0, 10)
+    far["origin"] -= far["direction"] * np.float32(1e5)
+    check(mesh_scene(v), far)
+
+
+def test_boxes_past_the_range_and_odd_rays(check):
+    v = soup(300, 11)
+    assert check(mesh_scene(v * np.float32(1e9)), hard_rays(v.reshape(-1, 3) * 1e9, 1e9, 1))["usable"] == 0
+    rays = hard_rays(v.reshape(-1, 3), 1.0, 12, 64)
+    rays["direction"][0] = (0, 0, 0)
+    rays["direction"][1] = (np.nan, 0, 1)
+    rays["direction"][2] = (np.inf, 0, 1)
+    rays["origin"][3] = (np.nan, 0, 0)
+    rays["origin"][4] = (0, np.inf, 0)
+    check(mesh_scene(v), rays)
+
+
+def test_instances_spheres_and_direct_lists(check):
+    rng = np.random.default_rng(2)
+    v = soup(400, 13, flat=True)
+    inst = [scenes.instance(0, rng.uniform(-4, 4, 3), s, 360 * rng.random())
+            for s in (1e-7, 1e-3, 0.3, 1.0, 1.0, 2.0, 7.0)] + [scenes.instance(0), scenes.instance(0)]
+    s = mesh_scene(v, *inst)
+    sp = np.zeros(60, abi.SPHERE_DTYPE)
+    sp["center"], sp["radius"] = rng.uniform(-4, 4, (60, 3)), rng.uniform(0.05, 0.8, 60)
+    sp["accel"] = np.where(np.arange(60) % 9 == 0, abi.ACCEL_DIRECT, abi.ACCEL_BVH)
+    sp[40:50] = sp[10:20]                                         # coincident spheres
+    s.spheres = sp
+    w = soup(30, 14)
+    s.static_triangles = scenes.triangles(w[:, 0], w[:, 1], w[:, 2], 0)
+    s.triangles = scenes.triangles(w[:, 0] + 1, w[:, 1] + 1, w[:, 2] + 1, 0)
+    got = check(s, hard_rays(np.concatenate([v.reshape(-1, 3), sp["center"]]), 4.0, 15, 20000))
+    assert got["redone"] > 0
+    only = Scene()
+    only.add_material(material(abi.MAT_DIFFUSE, (0.5, 0.5, 0.5)))
+    only.triangles = scenes.triangles(v[:, 0], v[:, 1], v[:, 2], 0)  # the direct list's own BVH
+    check(only, hard_rays(v.reshape(-1, 3), 1.0, 16, 8000))
+
+
+def test_repository_scenes(check):
+    rng = np.random.default_rng(4)
+    for scene, _ in (scenes.cornell_box(64, 64), scenes.textured_room(64, 64),
+                     scenes.sphere_field(64, 36, frequency=20),
+                     scenes.large_mesh(64, 36, terrain_quads=64, instance_count=20, instance_frequency=10,
+                                       glass_spheres=4, env_size=(64, 32))):
+        o = rng.uniform(-2, 3, (8000, 3)).astype(np.float32)
+        d = rng.normal(0, 1, (8000, 3)).astype(np.float32)
+        got = check(scene, make_rays(o, d / np.linalg.norm(d, axis=1, keepdims=True)))
+        # the Cornell box's boxes stand on its floor: rays from below meet both
+        assert got["redone"] < got["rays"] // 50 and got["wide_visits"] < 0.6 * got["binary_visits"], got

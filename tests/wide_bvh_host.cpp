@@ -1,0 +1,162 @@
+// Host build of the wide BVH's construction and traversal (wf_wide_build.cuh,
+// wf_wide.cuh) for tests/test_wide_bvh.py: every ray of a batch is traced by
+// the wide traversal and by the BVH2 traversal of the same scene.
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+#include <vector>
+
+#include <cuda_runtime.h>
+
+static inline uint32_t __float_as_uint(float f) { uint32_t u; std::memcpy(&u, &f, 4); return u; }
+static inline float __uint_as_float(uint32_t u) { float f; std::memcpy(&f, &u, 4); return f; }
+static inline int __float_as_int(float f) { return int(__float_as_uint(f)); }
+static inline float __int_as_float(int i) { return __uint_as_float(uint32_t(i)); }
+template <typename T> static inline T __ldg(const T* p) { return *p; }
+static inline float __fmaf_rn(float a, float b, float c) { return std::fma(a, b, c); }
+static inline int __popc(unsigned v) { return __builtin_popcount(v); }
+static inline int __ffs(int v) { return __builtin_ffs(v); }
+static inline int __clz(int v) { return v ? __builtin_clz(unsigned(v)) : 32; }
+static inline unsigned __activemask() { return 1u; }
+static inline bool __any_sync(unsigned, bool p) { return p; }
+static inline uint32_t __byte_perm(uint32_t x, uint32_t y, uint32_t s) {
+    uint64_t both = uint64_t(y) << 32 | x;
+    uint32_t r = 0;
+    for (int k = 0; k < 4; ++k) r |= uint32_t(both >> (8 * (s >> (4 * k) & 7u)) & 0xffu) << (8 * k);
+    return r;
+}
+using std::isfinite;
+using std::max;
+using std::min;
+
+#include "wf_internal.h"
+#include "wf_bvh_gpu.h"
+#include "wf_wide.cuh"
+#include "wf_wide_build.cuh"
+
+namespace wf {
+bool build_binary_bvh_gpu(const BvhBox*, uint32_t, std::vector<BvhBinaryNode>&, int, char*, size_t, int) {
+    return false;
+}
+}  // namespace wf
+
+using namespace wf;
+
+namespace {
+struct Built {
+    HostScene h;
+    DeviceScene v{};
+    std::vector<WideNode> nodes;
+    std::vector<WideTriangle> triangles;
+    std::vector<WideLeaf> leaves;
+};
+
+void build_wide(Built& b) {
+    std::vector<BvhRef> trees;
+    auto number = [&](BvhRef& r) {
+        if (r.root == kNoRoot) return;
+        r.wide = uint32_t(trees.size());
+        trees.push_back(r);
+    };
+    for (Blas& x : b.h.blases) number(x.bvh);
+    number(b.h.direct_bvh);
+    number(b.h.tlas);
+    std::vector<uint32_t> items;
+    for (uint32_t i = 0; i < trees.size(); ++i) {
+        uint32_t item = trees[i].root < 0 ? (kLeafItem | uint32_t(~trees[i].root)) : uint32_t(trees[i].root);
+        items.push_back(item | (i == b.h.tlas.wide ? kTlasItem : 0u));
+    }
+    bool usable = true;
+    std::vector<uint2> bases;
+    uint32_t triangle_count = 0, leaf_count = 0;
+    for (uint32_t i = 0; i < items.size(); ++i) {
+        Collapsed c;
+        collapse(b.h.nodes.data(), items[i], trees.data() + i, c);
+        bool tlas = (items[i] & kTlasItem) != 0;
+        uint32_t& entries = tlas ? leaf_count : triangle_count;
+        bases.push_back(make_uint2(uint32_t(items.size()), entries));
+        entries += uint32_t(c.leaves);
+        for (int k = 0; k < kWide; ++k) {
+            if (c.count[k] == 0) continue;
+            for (int a = 0; a < 3; ++a)
+                usable = usable && std::fabs(c.child[k].lo[a]) <= kWideMaxCoordinate &&
+                         std::fabs(c.child[k].hi[a]) <= kWideMaxCoordinate;
+            if (c.count[k] < 0) items.push_back(uint32_t(c.child[k].ref) | (tlas ? kTlasItem : 0u));
+        }
+    }
+    DeviceScene& v = b.v;
+    v.triangles = b.h.triangles.data();
+    v.nodes = b.h.nodes.data();
+    v.blases = b.h.blases.data();
+    v.instances = b.h.instances.data();
+    v.mesh_linear = b.h.mesh_linear.data();
+    v.tlas_leaves = b.h.tlas_leaves.data();
+    v.spheres = b.h.spheres.data();
+    v.direct_spheres = b.h.direct_spheres.data();
+    v.direct_instances = b.h.direct_instances.data();
+    v.materials = b.h.materials.data();
+    v.material_textures = b.h.material_textures.empty() ? nullptr : b.h.material_textures.data();
+    v.texels = b.h.texels.data();
+    v.textures = b.h.textures.data();
+    v.tri_attr = b.h.tri_attr.empty() ? nullptr : b.h.tri_attr.data();
+    v.texture_count = uint32_t(b.h.textures.size());
+    v.tlas = b.h.tlas;
+    v.direct_bvh = b.h.direct_bvh;
+    v.static_first = b.h.static_first;
+    v.static_count = b.h.static_count;
+    v.direct_first = b.h.direct_first;
+    v.direct_count = b.h.direct_count;
+    v.direct_sphere_count = uint32_t(b.h.direct_spheres.size());
+    v.direct_instance_count = uint32_t(b.h.direct_instances.size());
+    v.any_alpha_reject = b.h.any_alpha_reject ? 1u : 0u;
+    b.triangles.resize(triangle_count);
+    b.leaves.resize(leaf_count);
+    for (uint32_t i = 0; i < items.size(); ++i) {
+        Collapsed c;
+        collapse(v.nodes, items[i], trees.data() + i, c);
+        b.nodes.push_back(wide_record(v, c, (items[i] & kTlasItem) != 0, bases[i].x, bases[i].y, b.triangles.data(),
+                                      b.leaves.data()));
+    }
+    v.wide = WideBvh{b.nodes.data(), b.triangles.data(), b.leaves.data(), usable && !trees.empty() ? 1u : 0u};
+}
+}  // namespace
+
+// counts: [0] closest hits that differ, [1] occlusion answers that differ,
+// [2] rays, [3] wide nodes, [4] wide node visits, [5] BVH2 node visits,
+// [6] usable, [7] rays that the BVH2s decided, [8] hits
+extern "C" int wide_check(const wf_scene_desc* desc, const wf_ray* rays, const float* limits, uint32_t count,
+                          uint64_t* counts) {
+    Built b;
+    if (wf_status e = build_host_scene(desc, b.h)) return int(e);
+    build_wide(b);
+    for (int k = 0; k < 9; ++k) counts[k] = 0;
+    counts[2] = count;
+    counts[3] = b.nodes.size();
+    counts[6] = b.v.wide.usable;
+    for (uint32_t i = 0; i < count; ++i) {
+        V3 o{rays[i].origin[0], rays[i].origin[1], rays[i].origin[2]};
+        V3 d{rays[i].direction[0], rays[i].direction[1], rays[i].direction[2]};
+        CountTally steps, wide, wide_any, binary, unused;
+        TraceState x, y;
+        Lane lane;
+        StateSink sink;
+        lane_begin<false>(lane, b.v, sink, o, d, 1e30f, steps);
+        while (!lane_done(lane)) lane_step<false>(lane, b.v, sink, steps);
+        if (lane_doubt(lane)) ++counts[7];
+        x = trace_closest(b.v, o, d, wide);
+        y = trace_closest_binary(b.v, o, d, binary);
+        // u and v mean something for triangles only, the instance for meshes
+        uint32_t kind = hit_kind(y.prim);
+        bool triangle = kind == kHitMesh || kind == kHitTriangle;
+        if (x.prim != y.prim || std::memcmp(&x.t, &y.t, triangle ? 12 : 4) != 0 ||
+            (kind == kHitMesh && x.inst != y.inst))
+            ++counts[0];
+        if (kind != kHitMiss) ++counts[8];
+        bool p = trace_any(b.v, o, d, limits[i], wide_any), q = trace_any_binary(b.v, o, d, limits[i], unused);
+        if (p != q) ++counts[1];
+        counts[4] += wide.nodes;
+        counts[5] += binary.nodes;
+    }
+    return 0;
+}

@@ -134,8 +134,8 @@ WF_DEV void flush_vertex(uint32_t key, float4 value, float4* warp_buffer, const 
 // delta * dU/dtheta to the gradients and returns the replayed radiance.  In
 // adjoint mode all 32 lanes of the warp call it together (`alive` false for
 // lanes without a path) and run the same number of vertex steps.
-// Tally: the traversal variant (Opaque<NoTally> when no material of the scene
-// is alpha-textured, which drops the per-candidate alpha test).
+// Tally: the traversal variant (Opaque<NoTally> for scenes that allow it,
+// wf_scene::opaque).
 template <bool kAdjoint, typename Tally>
 WF_DEV V3 diff_path(const DeviceScene& s, const DiffParams& P, const DiffSettings& cfg, uint32_t px, uint32_t py,
                     uint32_t sample, bool alive, V3 total, V3 delta, const DiffGrads& G, float4* warp_buffer,
@@ -159,8 +159,7 @@ WF_DEV V3 diff_path(const DeviceScene& s, const DiffParams& P, const DiffSetting
         do {
             if (!alive) break;
             alive = false;  // set again below when the path continues
-            TraceState h;
-            trace_closest(s, o, d, h, tally);
+            TraceState h = trace_closest_call(s, o, d, tally);
             SurfaceHit sh;
             if (!finish_hit(s, o, d, h.t, h.u, h.v, h.prim, h.inst, sh)) break;
             const Material& m = s.materials[sh.material];
@@ -201,7 +200,7 @@ WF_DEV V3 diff_path(const DeviceScene& s, const DiffParams& P, const DiffSetting
                     V3 st = offset_ray_origin(lp, light.normal, -wl, dist);
                     V3 seg = st - so;
                     float sd = length(seg);
-                    if (sd > kRayMinDistance && !trace_any(s, so, seg / sd, sd - kRayMinDistance, tally)) {
+                    if (sd > kRayMinDistance && !trace_any_call(s, so, seg / sd, sd - kRayMinDistance, tally)) {
                         OrenNayar on = oren_nayar(n, wo, wl, sigma);
                         float geometry = cos_l * light.area / (dist2 * light.selection_pdf);
                         const Material& lm = s.materials[light.material];
@@ -369,7 +368,7 @@ extern "C" wf_status wf_diff_forward(const wf_scene* scene, const wf_camera* cam
     cudaError_t ce = cudaMemsetAsync(error, 0, sizeof(uint32_t), st);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync");
     DiffParams P{albedo, roughness, emission_scale};
-    if (scene->alpha_textures)
+    if (!scene->opaque())
         k_diff_forward<NoTally><<<diff_grid(cfg.w * cfg.h), 128, 0, st>>>(scene->view, P, cfg, image, error);
     else
         k_diff_forward<Opaque<NoTally>><<<diff_grid(cfg.w * cfg.h), 128, 0, st>>>(scene->view, P, cfg, image, error);
@@ -394,7 +393,7 @@ extern "C" wf_status wf_diff_backward(const wf_scene* scene, const wf_camera* ca
     DiffGrads G{d_albedo, d_roughness, d_emission_scale};
     uint32_t items = cfg.w * cfg.h * ((cfg.spp + 31) / 32);  // one warp each
     uint32_t blocks = std::max(1u, std::min((items + 3) / 4, 148u * 16u));
-    if (scene->alpha_textures)
+    if (!scene->opaque())
         k_diff_backward<NoTally><<<blocks, 128, 0, st>>>(scene->view, P, cfg, d_image, G, error);
     else
         k_diff_backward<Opaque<NoTally>><<<blocks, 128, 0, st>>>(scene->view, P, cfg, d_image, G, error);

@@ -16,7 +16,6 @@
 // batch of more units than one pass holds (the radiance buffer's size) runs
 // as several passes in unit order.
 #include "wf_wavefront.cuh"
-#include "wf_lane_traverse.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -56,7 +55,7 @@ struct BatchView {
 struct wf_batch {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
-    bool opaque = true;     // no job's scene has alpha-textured materials: the Opaque<> trace and shadow kernels
+    bool opaque = true;     // every job's scene is (wf_scene::opaque): the Opaque<> trace and shadow kernels
     bool textured = false;  // some job's scene has textured materials: k_batch_shade<true>
     int device = 0, sm_count = 148;
     std::vector<void*> allocations;
@@ -75,6 +74,7 @@ struct wf_batch {
     float4* shadow_origin = nullptr;
     float4* shadow_dir = nullptr;
     uint8_t* shadow_result = nullptr;
+    uint32_t* shadow_chain = nullptr;  // requests left to the BVH2s (k_batch_shadow)
     uint32_t shadow_capacity = 0;
     wf::Counters* counters = nullptr;
     uint32_t capacity = 0, units = 0, pass_units = 0, block = 128, refill = 8, max_depth = 1;
@@ -165,7 +165,7 @@ __global__ void k_batch_accumulate(BatchView b, const Counters* c) {
 
 // At most 72 registers, as k_trace (7 CTAs of 128 per SM instead of 6).
 template <typename Tally>
-__global__ void __maxnreg__(72) k_batch_trace(BatchView b, PathSoA ps, const uint32_t* queue, const uint32_t* count, float4* hit_a,
+__global__ void __maxnreg__(64) k_batch_trace(BatchView b, PathSoA ps, const uint32_t* queue, const uint32_t* count, float4* hit_a,
                               uint32_t* hit_inst, Counters* c, uint32_t refill_at) {
     count_launch(c);
     uint32_t n = *count;
@@ -177,36 +177,46 @@ __global__ void __maxnreg__(72) k_batch_trace(BatchView b, PathSoA ps, const uin
         c->extension_rays += n;
     }
     Tally tally;
-    ClosestLane L;
-    L.stage = kStageDone;
+    Lane L;
+    L.state = kStageDone;
     const DeviceScene* sp = nullptr;
-    uint32_t i = 0;
+    QueueSink sink{hit_a, hit_inst, 0};
+    uint32_t doubts = kInvalid;
     RayFeed feed;
     uint32_t slot = feed_begin(feed, n);
-    for (;; slot = feed_next(feed, &c->work_trace, L.stage == kStageDone, refill_at)) {
-        if (slot != kInvalid) {
-            i = slot;
-            uint32_t p = queue[i];
+    for (;; slot = feed_next(feed, &c->work_trace, lane_done(L), refill_at)) {
+        bool busy = slot != kInvalid;
+        if (busy) {
+            sink.i = slot;
+            uint32_t p = queue[sink.i];
             sp = &b.jobs[b.slot_job[p]].scene;
             float4 o = ps.origin[p], d = ps.direction[p];
-            closest_begin(L, *sp, f4xyz(o), f4xyz(d), tally);
-            if (L.stage == kStageDone) {
-                hit_a[i] = make_float4(L.h.t, L.h.u, L.h.v, __uint_as_float(L.h.prim));
-                hit_inst[i] = L.h.inst;
-            }
+            lane_begin<false>(L, *sp, sink, f4xyz(o), f4xyz(d), 1e30f, tally);
         }
-        bool busy = L.stage != kStageDone;
+        busy = busy || !lane_done(L);
         if (!__any_sync(0xffffffffu, busy)) {
             if (!feed.more) break;
             continue;
         }
         if (busy) {
-            closest_step(L, *sp, tally);
-            if (L.stage == kStageDone) {
-                hit_a[i] = make_float4(L.h.t, L.h.u, L.h.v, __uint_as_float(L.h.prim));
-                hit_inst[i] = L.h.inst;
+            if (!lane_done(L)) lane_step<false>(L, *sp, sink, tally);
+            if (lane_done(L)) {
+                lane_finish<false>(L, *sp, sink, tally);
+                if (lane_doubt(L)) {
+                    hit_inst[sink.i] = doubts;
+                    doubts = sink.i;
+                }
             }
         }
+    }
+    // rays for the BVH2s, chained through their instance words
+    while (doubts != kInvalid) {
+        uint32_t i = doubts, p = queue[i];
+        doubts = hit_inst[i];
+        float4 o = ps.origin[p], d = ps.direction[p];
+        TraceState h = trace_closest_binary(b.jobs[b.slot_job[p]].scene, f4xyz(o), f4xyz(d), tally);
+        hit_a[i] = make_float4(h.t, h.u, h.v, __uint_as_float(h.prim));
+        hit_inst[i] = h.inst;
     }
 }
 
@@ -255,36 +265,51 @@ __global__ void __launch_bounds__(128, 4) k_batch_shade(BatchView b, PathSoA ps,
 }
 
 template <typename Tally>
-__global__ void k_batch_shadow(BatchView b, const float4* shadow_origin, const float4* shadow_dir, uint8_t* result,
-                               Counters* c, uint32_t capacity, uint32_t refill_at) {
+__global__ void __maxnreg__(64) k_batch_shadow(BatchView b, const float4* shadow_origin, const float4* shadow_dir, uint8_t* result,
+                               uint32_t* chain, Counters* c, uint32_t capacity, uint32_t refill_at) {
     count_launch(c);
     uint32_t n = min(c->shadow_count, capacity);
     uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid == 0) c->shadow_rays += n;
     Tally tally;
-    AnyLane L;
-    L.stage = kStageDone;
+    Lane L;
+    L.state = kStageDone;
     const DeviceScene* sp = nullptr;
-    uint32_t j = 0;
+    uint32_t j = 0, doubts = kInvalid;
+    NoSink sink;
     RayFeed feed;
     uint32_t slot = feed_begin(feed, n);
-    for (;; slot = feed_next(feed, &c->work_shadow, L.stage == kStageDone, refill_at)) {
-        if (slot != kInvalid) {
+    for (;; slot = feed_next(feed, &c->work_shadow, lane_done(L), refill_at)) {
+        bool busy = slot != kInvalid;
+        if (busy) {
             j = slot;
             float4 o = shadow_origin[j], d = shadow_dir[j];
             sp = &b.jobs[__float_as_uint(d.w)].scene;
-            any_begin(L, *sp, f4xyz(o), f4xyz(d), o.w, tally);
-            if (L.stage == kStageDone) result[j] = L.hit ? 1 : 0;
+            lane_begin<true>(L, *sp, sink, f4xyz(o), f4xyz(d), o.w, tally);
         }
-        bool busy = L.stage != kStageDone;
+        busy = busy || !lane_done(L);
         if (!__any_sync(0xffffffffu, busy)) {
             if (!feed.more) break;
             continue;
         }
         if (busy) {
-            any_step(L, *sp, tally);
-            if (L.stage == kStageDone) result[j] = L.hit ? 1 : 0;
+            if (!lane_done(L)) lane_step<true>(L, *sp, sink, tally);
+            if (lane_done(L)) {
+                lane_finish<true>(L, *sp, sink, tally);
+                if (lane_doubt(L)) {
+                    chain[j] = doubts;
+                    doubts = j;
+                } else {
+                    result[j] = (L.state & kHit) ? 1 : 0;
+                }
+            }
         }
+    }
+    while (doubts != kInvalid) {  // rays for the BVH2s
+        uint32_t i = doubts;
+        doubts = chain[i];
+        float4 o = shadow_origin[i], d = shadow_dir[i];
+        result[i] = trace_any_binary(b.jobs[__float_as_uint(d.w)].scene, f4xyz(o), f4xyz(d), o.w, tally) ? 1 : 0;
     }
 }
 
@@ -447,11 +472,11 @@ wf_status capture_batch(wf_batch* b) {
                 b->shadow_origin, b->shadow_dir, b->shadow_capacity, b->counters, next_count);
         if (b->opaque)
             k_batch_shadow<Opaque<NoTally>><<<batch_grid(b, 2, b->shadow_capacity, b->block), b->block, 0, st>>>(
-                b->view, b->shadow_origin, b->shadow_dir, b->shadow_result, b->counters, b->shadow_capacity,
+                b->view, b->shadow_origin, b->shadow_dir, b->shadow_result, b->shadow_chain, b->counters, b->shadow_capacity,
                 b->refill);
         else
             k_batch_shadow<NoTally><<<batch_grid(b, 2, b->shadow_capacity, b->block), b->block, 0, st>>>(
-                b->view, b->shadow_origin, b->shadow_dir, b->shadow_result, b->counters, b->shadow_capacity,
+                b->view, b->shadow_origin, b->shadow_dir, b->shadow_result, b->shadow_chain, b->counters, b->shadow_capacity,
                 b->refill);
         k_batch_finalize<<<batch_grid(b, 3, cap, 256), 256, 0, st>>>(
             b->view, b->paths, b->queue[cur], cur_count, b->terms, b->shade_out, b->shadow_result, b->queue[nxt],
@@ -527,7 +552,7 @@ wf_status batch_create(const wf_batch_job* jobs, uint32_t count, const wf_batch_
     b->block = config.block_size ? config.block_size : 128u;
     b->refill = config.refill_threshold ? config.refill_threshold : 8u;
     for (uint32_t i = 0; i < count; ++i) {
-        b->opaque = b->opaque && !jobs[i].scene->alpha_textures;
+        b->opaque = b->opaque && jobs[i].scene->opaque();
         b->textured = b->textured || jobs[i].scene->textured;
     }
 
@@ -608,6 +633,7 @@ wf_status batch_create(const wf_batch_job* jobs, uint32_t count, const wf_batch_
     WF_BATCH_CUDA(batch_alloc(bp, &b->shadow_origin, b->shadow_capacity));
     WF_BATCH_CUDA(batch_alloc(bp, &b->shadow_dir, b->shadow_capacity));
     WF_BATCH_CUDA(batch_alloc(bp, &b->shadow_result, b->shadow_capacity));
+    WF_BATCH_CUDA(batch_alloc(bp, &b->shadow_chain, b->shadow_capacity));
     WF_BATCH_CUDA(batch_alloc(bp, &b->counters, 1));
     WF_BATCH_CUDA(cudaMemcpyAsync(b->jobs_dev, host.data(), sizeof(BatchJob) * count, cudaMemcpyHostToDevice,
                                   b->stream));

@@ -13,6 +13,7 @@
 #include <memory>
 
 #include "wf_renderer.h"
+#include "wf_wide_bvh.h"
 #include "wf_bvh_gpu.h"
 
 namespace wf {
@@ -163,6 +164,17 @@ wf_status wf_scene_create(const wf_scene_desc* desc, wf_scene** out) {
     auto up = [&](auto** dst, const auto& vec) {
         if (e == cudaSuccess) e = upload(s.get(), L, B, dst, vec);
     };
+    // Wide root i belongs to tree i of this list.
+    std::vector<BvhRef> trees;
+    auto number = [&](BvhRef& ref) {
+        if (ref.root == kNoRoot) return;
+        ref.wide = uint32_t(trees.size());
+        trees.push_back(ref);
+    };
+    for (Blas& b : h.blases) number(b.bvh);
+    number(h.direct_bvh);
+    number(h.tlas);
+    uint32_t tlas_tree = h.tlas.wide;
     up(&v.triangles, h.triangles);
     up(&v.normals, h.normals);
     up(&v.nodes, h.nodes);
@@ -181,6 +193,7 @@ wf_status wf_scene_create(const wf_scene_desc* desc, wf_scene** out) {
     up(&v.tri_attr, h.tri_attr);
     up(&v.lights, h.lights);
     up(&v.punctual, h.punctual);
+    if (e == cudaSuccess) e = build_wide_bvh(v, trees, uint32_t(h.nodes.size()), tlas_tree, L, B);
     if (e != cudaSuccess) {
         free_list(L);
         return e == cudaErrorMemoryAllocation ? fail(WF_ERR_OOM, "scene upload: out of device memory")

@@ -9,6 +9,9 @@
 //   * BVH2 nodes: 64 B, both child boxes stored in the parent
 //     (lxy | rxy | lrz | children), so one node visit is four 16-byte loads and
 //     tests two boxes.  Child refs >= 0 are node indices, < 0 are ~leaf.
+//   * wide nodes: the same trees collapsed to 8 children per 80-byte node with
+//     8-bit box planes; every traversal uses them, and the BVH2 nodes decide
+//     the rays whose result could depend on the visit order (wf_wide.cuh).
 //   * spheres: float4 (center, radius) + material.
 // The arithmetic helpers reproduce the reference's Vec3 operators
 // (include/core/vec3.cuh:6-99) operation for operation so that, compiled with
@@ -100,11 +103,60 @@ struct Box {
 };
 
 // One BVH: root ref (node index, or ~leaf when the tree is a single leaf,
-// or kNoRoot when empty) and the root box.
+// or kNoRoot when empty), the root box and the root's wide node.
 constexpr int kNoRoot = 0x7fffffff;
+constexpr uint32_t kNoWide = 0xffffffffu;
 struct BvhRef {
     int root;
     Box box;
+    uint32_t wide;  // wide node index of the root (kNoWide when empty)
+};
+
+// Compressed 8-wide node, after Ylitie, Karras and Laine, "Efficient
+// Incoherent Ray Traversal on GPUs Through Compressed Wide BVHs" (HPG 2017):
+// child boxes as 8-bit planes on a per-node grid (origin p, power-of-two cell
+// sizes), internal children and leaf entries each contiguous.
+//   scale: bytes 0-2 the biased exponent of 2^15 x the cell size per axis,
+//          byte 3 the mask of slots that hold internal children
+//   meta[slot]: 0 empty; internal: 0x20 | (24 + slot); leaf: count in unary
+//          (1, 3, 7) << 5 | first entry relative to leaf_base
+//   planes: lo x, lo y, lo z, hi x, hi y, hi z; 8 bytes each, by slot
+struct alignas(16) WideNode {
+    float px, py, pz;
+    uint32_t scale;
+    uint32_t child_base, leaf_base;
+    uint32_t meta[2];
+    uint32_t planes[12];
+};
+static_assert(sizeof(WideNode) == 80, "wide node must be 80 bytes");
+
+// Leaf entries of the wide triangle BVHs, in leaf order: v0, v1 - v0 and
+// v2 - v0 (the edges the intersection test starts with), .w = packed
+// triangle index, material, unused.
+struct alignas(16) WideTriangle {
+    float4 v0, e1, e2;
+};
+
+// Leaf entries of the wide TLAS: everything an instance entry reads, in one
+// record.  `box` is the BVH2 leaf's box.
+struct alignas(16) WideLeaf {
+    float4 x, y, z;    // world-to-local rows, .w = translation; a sphere's (center, radius) in x
+    float4 lo;         // leaf box lo, .w = tlas_leaves word ((is_sphere << 31) | index)
+    float4 hi;         // leaf box hi, .w = wide root of the BLAS (kNoWide: none)
+    float4 root_lo;    // BLAS root box lo, .w = material override
+    float4 root_hi;    // BLAS root box hi, .w = BLAS index
+};
+static_assert(sizeof(WideLeaf) == 112, "TLAS leaf record");
+
+// The wide traversal's error bounds hold for coordinates up to this size
+// (wf_wide.cuh); larger scenes use the BVH2s alone.
+constexpr float kWideMaxCoordinate = 1.0e7f;
+
+struct WideBvh {
+    const WideNode* nodes;
+    const WideTriangle* triangles;
+    const WideLeaf* leaves;
+    uint32_t usable;  // 0: some box is not finite or beyond kWideMaxCoordinate
 };
 
 // Triangle .w lanes: a.w = original index | kTriHasNormals, b.w = material,
@@ -280,6 +332,7 @@ struct DeviceScene {
     const Light* lights;
     const Punctual* punctual;
     Environment env;
+    WideBvh wide;
     BvhRef tlas;
     BvhRef direct_bvh;  // direct-list triangle BVH (root kNoRoot = linear scan)
     uint32_t static_first, static_count;

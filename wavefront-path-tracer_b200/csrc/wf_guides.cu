@@ -49,9 +49,8 @@ WF_DEV bool project_frame_point(const Camera& c, V3 point, uint32_t width, uint3
 
 // The closest hit of one ray as a SurfaceHit; false on a miss.
 WF_DEV bool closest_surface(const DeviceScene& s, V3 o, V3 d, SurfaceHit& sh) {
-    TraceState h;
     NoTally tally;
-    trace_closest(s, o, d, h, tally);
+    TraceState h = trace_coherent(s, o, d, tally);
     return finish_hit(s, o, d, h.t, h.u, h.v, h.prim, h.inst, sh);
 }
 

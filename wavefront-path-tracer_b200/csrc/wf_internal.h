@@ -43,8 +43,8 @@ struct HostScene {
     std::vector<Light> lights;
     std::vector<Punctual> punctual;
     uint32_t directional_count = 0;
-    BvhRef tlas{kNoRoot, {}};
-    BvhRef direct_bvh{kNoRoot, {}};
+    BvhRef tlas{kNoRoot, {}, kNoWide};
+    BvhRef direct_bvh{kNoRoot, {}, kNoWide};
     uint32_t static_first = 0, static_count = 0;
     uint32_t direct_first = 0, direct_count = 0;
     bool any_alpha_reject = false;
@@ -96,6 +96,11 @@ struct wf_scene {
     uint32_t gpu_bvh_builds = 0;
     double bvh_build_ms = 0.0;
     bool alpha_textures = false;  // some material is alpha-masked with an albedo texture
+    // neither alpha-textured materials nor primitives outside the BVHs: the Opaque<> kernels
+    bool opaque() const {
+        return !alpha_textures && view.direct_instance_count == 0 && view.static_count == 0 &&
+               (view.direct_count == 0 || view.direct_bvh.root != wf::kNoRoot);
+    }
     bool textured = false;        // some material has a texture binding
     uint32_t material_categories = 0;  // bit k: some material has shading category k (material_category)
     wf::Box bounds{};

@@ -16,7 +16,6 @@
 // a bounded grid barrier between bounces.
 #include "wf_renderer.h"
 #include "wf_shade.cuh"
-#include "wf_lane_traverse.cuh"
 #include "wf_wavefront.cuh"
 
 #include <cuda.h>
@@ -153,42 +152,51 @@ WF_DEV void trace_stage(const DeviceScene& s, PathSoA ps, const uint32_t* queue,
             if (i >= first + n) continue;
             uint32_t p = queue[i];
             float4 o = ps.origin[p], d = ps.direction[p];
-            TraceState h;
-            trace_closest(s, f4xyz(o), f4xyz(d), h, tally);
+            TraceState h = trace_coherent(s, f4xyz(o), f4xyz(d), tally);
             hit_a[i] = make_float4(h.t, h.u, h.v, __uint_as_float(h.prim));
             hit_inst[i] = h.inst;
         }
         if constexpr (Tally::kCounts) flush_tally(tally, totals);
         return;
     }
-    ClosestLane L;
-    L.stage = kStageDone;
-    uint32_t i = 0;
+    Lane L;
+    L.state = kStageDone;
+    QueueSink sink{hit_a, hit_inst, 0};
+    uint32_t doubts = kInvalid;
     RayFeed feed;
     uint32_t slot = feed_begin(feed, n);
-    for (;; slot = feed_next(feed, counter, L.stage == kStageDone, refill_at)) {
-        if (slot != kInvalid) {
-            i = first + slot;
-            uint32_t p = queue[i];
+    for (;; slot = feed_next(feed, counter, lane_done(L), refill_at)) {
+        bool busy = slot != kInvalid;
+        if (busy) {
+            sink.i = first + slot;
+            uint32_t p = queue[sink.i];
             float4 o = ps.origin[p], d = ps.direction[p];
-            closest_begin(L, s, f4xyz(o), f4xyz(d), tally);
-            if (L.stage == kStageDone) {
-                hit_a[i] = make_float4(L.h.t, L.h.u, L.h.v, __uint_as_float(L.h.prim));
-                hit_inst[i] = L.h.inst;
-            }
+            lane_begin<false>(L, s, sink, f4xyz(o), f4xyz(d), 1e30f, tally);
         }
-        bool busy = L.stage != kStageDone;
+        busy = busy || !lane_done(L);
         if (!__any_sync(0xffffffffu, busy)) {
             if (!feed.more) break;
             continue;
         }
         if (busy) {
-            closest_step(L, s, tally);
-            if (L.stage == kStageDone) {
-                hit_a[i] = make_float4(L.h.t, L.h.u, L.h.v, __uint_as_float(L.h.prim));
-                hit_inst[i] = L.h.inst;
+            if (!lane_done(L)) lane_step<false>(L, s, sink, tally);
+            if (lane_done(L)) {
+                lane_finish<false>(L, s, sink, tally);
+                if (lane_doubt(L)) {
+                    hit_inst[sink.i] = doubts;
+                    doubts = sink.i;
+                }
             }
         }
+    }
+    // rays for the BVH2s, chained through their instance words
+    while (doubts != kInvalid) {
+        uint32_t i = doubts, p = queue[i];
+        doubts = hit_inst[i];
+        float4 o = ps.origin[p], d = ps.direction[p];
+        TraceState h = trace_closest_binary(s, f4xyz(o), f4xyz(d), tally);
+        hit_a[i] = make_float4(h.t, h.u, h.v, __uint_as_float(h.prim));
+        hit_inst[i] = h.inst;
     }
     if constexpr (Tally::kCounts) flush_tally(tally, totals);
 }
@@ -198,7 +206,7 @@ WF_DEV void trace_stage(const DeviceScene& s, PathSoA ps, const uint32_t* queue,
 // out; a 64-register cap spills far more.  __maxnreg__ keeps every block
 // size launchable.
 template <typename Tally, bool kLanes = true>
-__global__ void __maxnreg__(72) k_trace(DeviceScene s, PathSoA ps, const uint32_t* queue, const uint32_t* count,
+__global__ void __maxnreg__(64) k_trace(const __grid_constant__ DeviceScene s, PathSoA ps, const uint32_t* queue, const uint32_t* count,
                                         float4* hit_a, uint32_t* hit_inst, Counters* c, uint32_t bounce,
                                         TallyTotals* totals, uint32_t refill_at, const uint32_t* camera,
                                         uint32_t* work) {
@@ -210,7 +218,7 @@ __global__ void __maxnreg__(72) k_trace(DeviceScene s, PathSoA ps, const uint32_
 // more from the extra warps than its spills cost: bounce 0 of the 1080p large
 // mesh 2.07 -> 1.98 ms, the frame +0.6 %.
 template <typename Tally>
-__global__ void __launch_bounds__(128, 8) k_trace_camera(DeviceScene s, PathSoA ps, const uint32_t* queue,
+__global__ void __launch_bounds__(128, 8) k_trace_camera(const __grid_constant__ DeviceScene s, PathSoA ps, const uint32_t* queue,
                                                          const uint32_t* count, float4* hit_a, uint32_t* hit_inst,
                                                          Counters* c, uint32_t bounce, TallyTotals* totals,
                                                          uint32_t refill_at, const uint32_t* camera, uint32_t* work) {
@@ -396,38 +404,54 @@ __global__ void k_gather_dense(const __grid_constant__ RenderParams rp, GatherQu
 }
 
 template <typename Tally>
-WF_DEV void shadow_stage(DeviceScene s, const float4* shadow_origin, const float4* shadow_dir, uint8_t* result, Counters* c, uint32_t capacity, TallyTotals* totals, uint32_t refill_at) {
+WF_DEV void shadow_stage(const DeviceScene& s, const float4* shadow_origin, float4* shadow_dir, uint8_t* result, Counters* c, uint32_t capacity, TallyTotals* totals, uint32_t refill_at) {
     uint32_t n = min(c->shadow_count, capacity);
     uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid == 0) c->shadow_rays += n;
     Tally tally;
-    AnyLane L;
-    L.stage = kStageDone;
-    uint32_t j = 0;
+    Lane L;
+    L.state = kStageDone;
+    uint32_t j = 0, doubts = kInvalid;
+    NoSink sink;
     RayFeed feed;
     uint32_t slot = feed_begin(feed, n);
-    for (;; slot = feed_next(feed, &c->work_shadow, L.stage == kStageDone, refill_at)) {
-        if (slot != kInvalid) {
+    for (;; slot = feed_next(feed, &c->work_shadow, lane_done(L), refill_at)) {
+        bool busy = slot != kInvalid;
+        if (busy) {
             j = slot;
             float4 o = shadow_origin[j], d = shadow_dir[j];
-            any_begin(L, s, f4xyz(o), f4xyz(d), o.w, tally);
-            if (L.stage == kStageDone) result[j] = L.hit ? 1 : 0;
+            lane_begin<true>(L, s, sink, f4xyz(o), f4xyz(d), o.w, tally);
         }
-        bool busy = L.stage != kStageDone;
+        busy = busy || !lane_done(L);
         if (!__any_sync(0xffffffffu, busy)) {
             if (!feed.more) break;
             continue;
         }
         if (busy) {
-            any_step(L, s, tally);
-            if (L.stage == kStageDone) result[j] = L.hit ? 1 : 0;
+            if (!lane_done(L)) lane_step<true>(L, s, sink, tally);
+            if (lane_done(L)) {
+                lane_finish<true>(L, s, sink, tally);
+                if (lane_doubt(L)) {
+                    shadow_dir[j].w = __uint_as_float(doubts);
+                    doubts = j;
+                } else {
+                    result[j] = (L.state & kHit) ? 1 : 0;
+                }
+            }
         }
+    }
+    // rays for the BVH2s, chained through their requests' last words
+    while (doubts != kInvalid) {
+        uint32_t i = doubts;
+        float4 o = shadow_origin[i], d = shadow_dir[i];
+        doubts = __float_as_uint(d.w);
+        result[i] = trace_any_binary(s, f4xyz(o), f4xyz(d), o.w, tally) ? 1 : 0;
     }
     if constexpr (Tally::kCounts) flush_tally(tally, totals);
 }
 
 template <typename Tally>
-__global__ void k_shadow(DeviceScene s, const float4* shadow_origin, const float4* shadow_dir, uint8_t* result,
+__global__ void __maxnreg__(64) k_shadow(const __grid_constant__ DeviceScene s, const float4* shadow_origin, float4* shadow_dir, uint8_t* result,
                          Counters* c, uint32_t capacity, TallyTotals* totals, uint32_t refill_at) {
     count_launch(c);
     shadow_stage<Tally>(s, shadow_origin, shadow_dir, result, c, capacity, totals, refill_at);
@@ -684,9 +708,8 @@ __global__ void __launch_bounds__(128, 8) k_persistent(const __grid_constant__ D
                 if (i < n) {
                     p = cur[i];
                     Path path = load_path(ps, p);
-                    TraceState h;
                     Tally tally;
-                    trace_closest(s, path.origin, path.direction, h, tally);
+                    TraceState h = trace_closest_call(s, path.origin, path.direction, tally);
                     SurfaceHit sh;
                     bool did_hit = finish_hit(s, path.origin, path.direction, h.t, h.u, h.v, h.prim, h.inst, sh);
                     InlineSink<Tally> sink;
@@ -854,15 +877,15 @@ const void* phased_kernel(bool opaque, bool textured) {
 // One closest-hit traversal per thread, bounded to 8 CTAs of 128 per SM (64
 // registers; 68 unbounded): 4 M random rays against the 1080p large mesh,
 // 365 -> 388 Mrays/s.  k_any_batch already fits 8 CTAs (62 registers).
-__global__ void __launch_bounds__(128, 8) k_trace_batch(DeviceScene s, const wf_ray* rays, uint32_t count,
+template <typename Tally>
+__global__ void __launch_bounds__(128, 8) k_trace_batch(const __grid_constant__ DeviceScene s, const wf_ray* rays, uint32_t count,
                                                         wf_hit* hits) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     V3 o{rays[i].origin[0], rays[i].origin[1], rays[i].origin[2]};
     V3 d{rays[i].direction[0], rays[i].direction[1], rays[i].direction[2]};
-    TraceState h;
-    NoTally tally;
-    trace_closest(s, o, d, h, tally);
+    Tally tally;
+    TraceState h = trace_closest(s, o, d, tally);
     SurfaceHit sh;
     wf_hit out;
     memset(&out, 0, sizeof(out));
@@ -904,13 +927,14 @@ __global__ void __launch_bounds__(128, 8) k_trace_batch(DeviceScene s, const wf_
     hits[i] = out;
 }
 
-__global__ void k_any_batch(DeviceScene s, const wf_ray* rays, const float* max_distance, uint32_t count,
+template <typename Tally>
+__global__ void __launch_bounds__(128, 8) k_any_batch(const __grid_constant__ DeviceScene s, const wf_ray* rays, const float* max_distance, uint32_t count,
                             uint8_t* occluded) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     V3 o{rays[i].origin[0], rays[i].origin[1], rays[i].origin[2]};
     V3 d{rays[i].direction[0], rays[i].direction[1], rays[i].direction[2]};
-    NoTally tally;
+    Tally tally;
     occluded[i] = trace_any(s, o, d, max_distance[i], tally) ? 1 : 0;
 }
 
@@ -970,9 +994,8 @@ __global__ void __launch_bounds__(128, 8) k_trace_photons(const __grid_constant_
     uint32_t specular_bounces = 0;
     V3 o = f4xyz(p0), d = f4xyz(p1);
     for (uint32_t depth = 0; depth < max_depth; ++depth) {
-        TraceState h;
         NoTally tally;
-        trace_closest(s, o, d, h, tally);
+        TraceState h = trace_closest_call(s, o, d, tally);
         SurfaceHit hit;
         if (!finish_hit(s, o, d, h.t, h.u, h.v, h.prim, h.inst, hit)) return;
         if (hit.material >= s.material_count) return;
@@ -1210,8 +1233,8 @@ wf_status build_photon_map(wf_renderer* r) {
 }
 
 // k_trace / k_shadow for this renderer's scene: the Opaque<> variants (the
-// per-hit alpha-texture test compiled out, fewer registers) unless some
-// material of the scene is alpha-textured.
+// per-hit alpha-texture test and the linear primitive lists compiled out,
+// fewer registers) where the scene has neither (wf_scene::opaque).
 template <typename Tally, bool kLanes, typename... A>
 void launch_trace(const wf_renderer* r, uint32_t grid_size, uint32_t block, cudaStream_t st, A... args) {
     if constexpr (!kLanes) {
@@ -1546,7 +1569,7 @@ wf_status renderer_create_impl(const wf_scene* scene, const wf_camera* camera, c
     if (c.block_size) r->block_trace = c.block_size;
     r->refill = c.refill_threshold ? c.refill_threshold : 8u;
     r->regenerate_percent = c.regenerate_percent ? std::min(c.regenerate_percent, 100u) : kDefaultRegeneratePercent;
-    r->opaque = !scene->alpha_textures;
+    r->opaque = scene->opaque();
     r->textured = scene->textured;
     // Sorting by category pays only when hits can need different long
     // shading branches: with one of diffuse / metal / dielectric / other
@@ -2064,7 +2087,10 @@ wf_status renderer_profile(wf_renderer* r, wf_kernel_profile* out) {
 wf_status trace_closest_batch(const wf_scene* scene, const wf_ray* rays, uint32_t count, wf_hit* hits,
                               cudaStream_t stream) {
     if (count == 0) return WF_OK;
-    k_trace_batch<<<(count + 127) / 128, 128, 0, stream>>>(scene->view, rays, count, hits);
+    if (scene->opaque())
+        k_trace_batch<Opaque<NoTally>><<<(count + 127) / 128, 128, 0, stream>>>(scene->view, rays, count, hits);
+    else
+        k_trace_batch<NoTally><<<(count + 127) / 128, 128, 0, stream>>>(scene->view, rays, count, hits);
     WF_CUDA(cudaGetLastError());
     return WF_OK;
 }
@@ -2072,7 +2098,10 @@ wf_status trace_closest_batch(const wf_scene* scene, const wf_ray* rays, uint32_
 wf_status trace_any_batch(const wf_scene* scene, const wf_ray* rays, const float* max_distance, uint32_t count,
                           uint8_t* occluded, cudaStream_t stream) {
     if (count == 0) return WF_OK;
-    k_any_batch<<<(count + 127) / 128, 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
+    if (scene->opaque())
+        k_any_batch<Opaque<NoTally>><<<(count + 127) / 128, 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
+    else
+        k_any_batch<NoTally><<<(count + 127) / 128, 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
     WF_CUDA(cudaGetLastError());
     return WF_OK;
 }
@@ -2197,7 +2226,7 @@ extern "C" wf_status wf_render_tile_static(const wf_scene* scene, const wf_camer
     if (device < 0 || device >= kStaticMaxDevices) return fail(WF_ERR_UNSUPPORTED, "device index %d", device);
     unsigned char* base = nullptr;
     uint32_t resident = 0;
-    const bool opaque = !scene->alpha_textures;
+    const bool opaque = scene->opaque();
     const void* kernel = persistent_kernel(opaque, scene->textured);
     const int variant = !opaque ? 0 : (scene->textured ? 1 : 2);
     {

@@ -94,7 +94,7 @@ struct wf_renderer {
     wf::RenderParams params{};
     cudaStream_t stream = nullptr;
     bool own_stream = false;
-    bool opaque = true;     // no alpha-textured material: the Opaque<> trace and shadow kernels
+    bool opaque = true;     // wf_scene::opaque: the Opaque<> trace and shadow kernels
     bool textured = false;  // some textured material: k_shade<true>
     bool sort_shading = true;  // material-sort the hits before shading (k_classify, k_scatter)
     int device = 0;

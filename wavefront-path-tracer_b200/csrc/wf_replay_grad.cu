@@ -107,9 +107,8 @@ __global__ void __launch_bounds__(128, 8) k_albedo_gradient(const __grid_constan
             sink.grad = grad;
             sink.count = gp.count;
             for (uint32_t bounce = 0; bounce < rp.max_depth && bounce < kMaxBounces; ++bounce) {
-                TraceState h;
                 Tally tally;
-                trace_closest(s, path.origin, path.direction, h, tally);
+                TraceState h = trace_closest_call(s, path.origin, path.direction, tally);
                 SurfaceHit sh;
                 bool did_hit = finish_hit(s, path.origin, path.direction, h.t, h.u, h.v, h.prim, h.inst, sh);
                 sink.own = -1;

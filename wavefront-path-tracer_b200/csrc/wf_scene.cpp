@@ -93,7 +93,7 @@ struct Converter {
         return index;
     }
     BvhRef root() {
-        BvhRef ref{kNoRoot, {}};
+        BvhRef ref{kNoRoot, {}, kNoWide};
         if (bin.empty()) return ref;
         uint32_t r = uint32_t(bin.size() - 1);
         ref.box = to_box(bin[r].box);
@@ -397,7 +397,7 @@ wf_status build_host_scene(const wf_scene_desc* d, HostScene& s) {
     for (uint32_t m = 0; m < d->mesh_count; ++m) {
         const wf_mesh& mesh = d->meshes[m];
         Blas b{};
-        b.bvh = BvhRef{kNoRoot, {}};
+        b.bvh = BvhRef{kNoRoot, {}, kNoWide};
         b.first = uint32_t(s.triangles.size() / 3);
         b.count = mesh.triangle_count;
         b.first_linear = uint32_t(s.mesh_linear.size());

@@ -15,7 +15,7 @@
 // makes the deferral exact.
 #pragma once
 
-#include "wf_traverse.cuh"
+#include "wf_wide.cuh"
 
 namespace wf {
 
@@ -586,7 +586,7 @@ struct InlineSink {
     WF_DEV int request(V3 o, V3 d, float t_max) {
         ++requests;
         Tally tally;
-        return trace_any(*scene, o, d, t_max, tally) ? 1 : 0;
+        return trace_any_call(*scene, o, d, t_max, tally) ? 1 : 0;
     }
     WF_DEV bool may_be_visible(int handle) const { return handle == kUnconditional || handle == 0; }
     WF_DEV void term(V3 c, int handle) {

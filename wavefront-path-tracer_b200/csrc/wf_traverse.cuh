@@ -25,12 +25,15 @@ constexpr int kStackSize = 64;  // leaf depth <= kMaxBvhDepth (60) < 64
 // sphere and instance tests a traversal performs, for the algorithmic-byte
 // accounting of the profiling pass.
 // A tally type also fixes, at compile time, whether the traversal may meet
-// alpha-textured materials (kAlphaTextures): the default types handle every
-// scene; Opaque<T> compiles the per-hit texture test out, for kernels that
-// the host launches only on scenes without such materials.
+// alpha-textured materials (kAlphaTextures) or primitives outside the BVHs
+// (kLinearLists: direct instances, static triangles, a direct list without a
+// BVH): the default types handle every scene; Opaque<T> compiles both out,
+// for kernels that the host launches only on scenes without either
+// (wf_scene::opaque).
 struct NoTally {
     static constexpr bool kCounts = false;
     static constexpr bool kAlphaTextures = true;
+    static constexpr bool kLinearLists = true;
     WF_DEV void node() {}
     WF_DEV void triangle() {}
     WF_DEV void sphere() {}
@@ -39,6 +42,7 @@ struct NoTally {
 struct CountTally {
     static constexpr bool kCounts = true;
     static constexpr bool kAlphaTextures = true;
+    static constexpr bool kLinearLists = true;
     uint32_t nodes = 0, triangles = 0, spheres = 0, instances = 0;
     WF_DEV void node() { ++nodes; }
     WF_DEV void triangle() { ++triangles; }
@@ -48,6 +52,7 @@ struct CountTally {
 template <typename Base>
 struct Opaque : Base {
     static constexpr bool kAlphaTextures = false;
+    static constexpr bool kLinearLists = false;
 };
 
 struct TraceState {
@@ -506,9 +511,13 @@ WF_DEV bool tlas_any(const DeviceScene& s, V3 o, V3 d, float t_max, Tally& tally
     }
 }
 
-// traceRay, device_traversal.cuh:1115-1150 (visit order and sphere reset rules).
+// traceRay, device_traversal.cuh:1115-1150 (visit order and sphere reset
+// rules), on the BVH2s: for coherent rays, whose warps visit the same nodes
+// in lockstep, and (trace_closest_binary) for the few rays whose answer in
+// the wide traversal could depend on the visit order (wf_wide.cuh).
 template <typename Tally>
-WF_DEV void trace_closest(const DeviceScene& s, V3 o, V3 d, TraceState& h, Tally& tally) {
+WF_DEV TraceState trace_coherent(const DeviceScene& s, V3 o, V3 d, Tally& tally) {
+    TraceState h;
     trace_state_init(h, 1e30f);
     for (uint32_t i = 0; i < s.direct_sphere_count; ++i) sphere_closest(s, s.direct_spheres[i], o, d, h, tally);
     for (uint32_t i = 0; i < s.direct_instance_count; ++i) instance_closest(s, s.direct_instances[i], o, d, h, false, tally);
@@ -548,12 +557,18 @@ WF_DEV void trace_closest(const DeviceScene& s, V3 o, V3 d, TraceState& h, Tally
         }
         if (h.t < previous) h.sphere = kInvalid;
     }
+    return h;
+}
+
+template <typename Tally>
+WF_CALL TraceState trace_closest_binary(const DeviceScene& s, V3 o, V3 d, Tally& tally) {
+    return trace_coherent(s, o, d, tally);
 }
 
 // isOccluded, device_traversal.cuh:1035-1113.  A pure disjunction of
 // independent tests, so an early return at the first hit gives the same bit.
 template <typename Tally>
-WF_DEV bool trace_any(const DeviceScene& s, V3 o, V3 d, float t_max, Tally& tally) {
+WF_CALL bool trace_any_binary(const DeviceScene& s, V3 o, V3 d, float t_max, Tally& tally) {
     for (uint32_t i = 0; i < s.direct_sphere_count; ++i) {
         float t;
         tally.sphere();

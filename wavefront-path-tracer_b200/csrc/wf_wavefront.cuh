@@ -71,6 +71,52 @@ WF_DEV bool next_chunk(uint32_t* counter, uint32_t n, uint32_t& base) {
     return base < n;
 }
 
+// Hands the rays [0, n) of a launch to its lanes.  Each of the launch's W
+// warps uses `width` of its lanes, so that n rays occupy all W warps before
+// a second ray joins a warp: a warp's step costs the sum of its lanes'
+// divergent branches, so a few hundred late-bounce rays packed 32 to a warp
+// ran at ~2,000 cycles a step against ~600 for a ray that has a warp to
+// itself.  From n = 32 W on every lane is used.  The first ray of a lane is
+// assigned by position, without an atomic; later ones come from `counter`.
+// The feed keeps only n, the width and a flag in registers (the closest-hit
+// loop has none to spare); the rest is recomputed at the rare refills.
+struct RayFeed {
+    uint32_t n;
+    uint32_t width;  // lanes in use, 1 to 32 (0: no rays)
+    bool more;       // rays are left to hand out (warp-uniform)
+};
+
+WF_DEV uint32_t feed_warps() { return (gridDim.x * blockDim.x) >> 5; }
+
+// Starts the feed and returns this lane's first ray, or kInvalid.
+WF_DEV uint32_t feed_begin(RayFeed& f, uint32_t n) {
+    uint32_t warps = feed_warps();
+    f.n = n;
+    f.width = min(32u, (n + warps - 1) / warps);
+    f.more = warps * f.width < n;
+    uint32_t lane = threadIdx.x & 31;
+    uint32_t slot = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * f.width + lane;
+    return lane < f.width && slot < n ? slot : kInvalid;
+}
+
+// The next ray for this lane, or kInvalid: once `threshold` lanes of the
+// warp (or all) are idle, they take rays with one warp-aggregated atomic.
+// Rays are left only when the first deal used all 32 lanes of every warp.
+WF_DEV uint32_t feed_next(RayFeed& f, uint32_t* counter, bool idle, uint32_t threshold) {
+    if (!f.more) return kInvalid;
+    unsigned mask = __ballot_sync(0xffffffffu, idle);
+    uint32_t k = __popc(mask);
+    if (k == 0 || (k < threshold && k < 32u)) return kInvalid;
+    uint32_t lane = threadIdx.x & 31;
+    uint32_t base = 0;
+    if (lane == 0) base = feed_warps() * 32u + atomicAdd(counter, k);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (base + k >= f.n) f.more = false;
+    if (!idle) return kInvalid;
+    uint32_t slot = base + __popc(mask & ((1u << lane) - 1u));
+    return slot < f.n ? slot : kInvalid;
+}
+
 // Sums a thread's tally into per-launch totals (profiling pass only).
 WF_DEV void flush_tally(const CountTally& t, TallyTotals* totals) {
     unsigned long long v[4] = {t.nodes, t.triangles, t.spheres, t.instances};

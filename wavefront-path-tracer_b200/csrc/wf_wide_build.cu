@@ -1,0 +1,116 @@
+// Collapses the scene's BVH2s into compressed 8-wide nodes on the GPU.
+//
+// One thread per wide node, level by level: a wide node starts with the two
+// children of its BVH2 node and opens its largest internal child (by box
+// area) until it has eight; what is left of at most kLeafTriangles triangles
+// becomes a leaf child.  The first pass numbers the nodes (each node's
+// internal children are contiguous) and counts the leaf entries, the second
+// writes the nodes, the triangles in leaf order and the TLAS leaf records, so
+// no array is larger than it has to be.  Bound by the random reads of the
+// BVH2 nodes (64 B each, read twice per pass at most).
+#include "wf_wide_bvh.h"
+#include "wf_renderer.h"
+#include "wf_wide_build.cuh"
+
+#include <algorithm>
+#include <cmath>
+
+namespace wf {
+namespace {
+
+// counters: [0] nodes, [1] triangles, [2] TLAS leaves, [3] boxes out of range
+__global__ void k_wide_number(const BvhNode* nodes, const BvhRef* roots, uint32_t begin, uint32_t end,
+                              uint32_t* items, uint2* bases, uint32_t* counters) {
+    uint32_t i = begin + blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= end) return;
+    uint32_t item = items[i];
+    bool tlas = (item & kTlasItem) != 0;
+    Collapsed c;
+    collapse(nodes, item, roots + i, c);
+    uint32_t base = c.internal ? atomicAdd(&counters[0], uint32_t(c.internal)) : 0u;
+    uint32_t leaf_base = c.leaves ? atomicAdd(&counters[tlas ? 2 : 1], uint32_t(c.leaves)) : 0u;
+    bases[i] = make_uint2(base, leaf_base);
+    bool fits = true;
+    for (int slot = 0; slot < kWide; ++slot) {
+        if (c.count[slot] == 0) continue;
+        for (int a = 0; a < 3; ++a)
+            fits = fits && fabsf(c.child[slot].lo[a]) <= kWideMaxCoordinate &&
+                   fabsf(c.child[slot].hi[a]) <= kWideMaxCoordinate;
+        if (c.count[slot] < 0) items[base++] = uint32_t(c.child[slot].ref) | (tlas ? kTlasItem : 0u);
+    }
+    if (!fits) counters[3] = 1u;
+}
+
+__global__ void k_wide_emit(DeviceScene s, const BvhRef* roots, uint32_t count, const uint32_t* items,
+                            const uint2* bases, WideNode* out, WideTriangle* triangles, WideLeaf* leaves) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    Collapsed c;
+    collapse(s.nodes, items[i], roots + i, c);
+    out[i] = wide_record(s, c, (items[i] & kTlasItem) != 0, bases[i].x, bases[i].y, triangles, leaves);
+}
+
+}  // namespace
+
+cudaError_t build_wide_bvh(DeviceScene& view, const std::vector<BvhRef>& roots, uint32_t node_count,
+                           uint32_t tlas_root, std::vector<void*>& allocations, uint64_t& bytes) {
+    view.wide = WideBvh{};
+    if (roots.empty()) return cudaSuccess;
+    uint32_t root_count = uint32_t(roots.size());
+    // Wide nodes other than the roots stand for distinct internal BVH2 nodes.
+    size_t capacity = size_t(node_count) + root_count;
+    uint32_t *items = nullptr, *counters = nullptr;
+    uint2* bases = nullptr;
+    BvhRef* root_refs = nullptr;
+    cudaError_t e = device_alloc(reinterpret_cast<void**>(&items), capacity * sizeof(uint32_t));
+    if (e == cudaSuccess) e = device_alloc(reinterpret_cast<void**>(&bases), capacity * sizeof(uint2));
+    if (e == cudaSuccess) e = device_alloc(reinterpret_cast<void**>(&counters), 4 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = device_alloc(reinterpret_cast<void**>(&root_refs), root_count * sizeof(BvhRef));
+    uint32_t host[4] = {root_count, 0, 0, 0};
+    if (e == cudaSuccess) {
+        std::vector<uint32_t> first(root_count);
+        for (uint32_t i = 0; i < root_count; ++i) {
+            first[i] = roots[i].root < 0 ? (kLeafItem | uint32_t(~roots[i].root)) : uint32_t(roots[i].root);
+            if (i == tlas_root) first[i] |= kTlasItem;
+        }
+        e = cudaMemcpy(items, first.data(), root_count * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(counters, host, sizeof(host), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = cudaMemcpy(root_refs, roots.data(), root_count * sizeof(BvhRef), cudaMemcpyHostToDevice);
+    uint32_t begin = 0;
+    while (e == cudaSuccess && begin < host[0]) {  // one level of all trees at a time
+        uint32_t end = host[0];
+        k_wide_number<<<(end - begin + 127) / 128, 128>>>(view.nodes, root_refs, begin, end, items, bases, counters);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaMemcpy(host, counters, sizeof(host), cudaMemcpyDeviceToHost);
+        begin = end;
+    }
+    WideNode* nodes = nullptr;
+    WideTriangle* triangles = nullptr;
+    WideLeaf* leaves = nullptr;
+    auto keep = [&](auto** p, size_t count) {
+        if (e != cudaSuccess) return;
+        size_t n = sizeof(**p) * std::max<size_t>(count, 1);
+        e = device_alloc(reinterpret_cast<void**>(p), n);
+        if (e != cudaSuccess) return;
+        allocations.push_back(*p);
+        bytes += n;
+    };
+    keep(&nodes, host[0]);
+    keep(&triangles, host[1]);
+    keep(&leaves, host[2]);
+    if (e == cudaSuccess) {
+        k_wide_emit<<<(host[0] + 127) / 128, 128>>>(view, root_refs, host[0], items, bases, nodes, triangles, leaves);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    cudaFree(items);
+    cudaFree(bases);
+    cudaFree(counters);
+    cudaFree(root_refs);
+    if (e == cudaSuccess) view.wide = WideBvh{nodes, triangles, leaves, host[3] ? 0u : 1u};
+    return e;
+}
+
+}  // namespace wf
