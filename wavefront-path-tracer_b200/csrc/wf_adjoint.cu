@@ -22,6 +22,9 @@
 //   dU/dtheta(t_m) += (U - P_m) * (dw_m/dtheta) / w_m + T_m * (df_m/dtheta) / f_m.
 // The adjoint kernel replays each path twice from its RNG key (pass A: U;
 // pass B: the sum above), instead of storing paths: memory is O(pixels).
+// Pass B takes the closest hits and light visibilities of the first
+// kReplayVertices vertices from a per-thread record of pass A and traces
+// only the deeper ones.
 // Gradients are accumulated with double atomics.
 #include "wf_wavefront.cuh"
 
@@ -128,6 +131,32 @@ WF_DEV void flush_vertex(uint32_t key, float4 value, float4* warp_buffer, const 
     __syncwarp();
 }
 
+// What pass A leaves for pass B: the closest hits of the first vertices and
+// whether their light samples were visible (20 bytes a vertex, in local
+// memory; the inverse-rendering configuration's paths have 6).
+constexpr uint32_t kReplayVertices = 8;
+struct PathRecord {
+    float4 hit[kReplayVertices];  // t, u, v, primitive
+    uint32_t inst[kReplayVertices];
+    uint32_t occluded;            // bit per vertex
+};
+
+// Lanes of a warp as (pixel, sample) pairs: 32 / spp pixels of spp samples
+// each, or one pixel's samples in chunks of 32.  Samples of one pixel meet
+// the same triangles, and the lanes of a pixel add up in sample order.
+struct DiffLanes {
+    uint32_t pixels;   // pixels per warp
+    uint32_t samples;  // samples per pixel and chunk
+    uint32_t chunks;
+};
+WF_HDI DiffLanes diff_lanes(uint32_t spp) {
+    DiffLanes l;
+    l.samples = spp < 32u ? spp : 32u;
+    l.pixels = 32u / l.samples;
+    l.chunks = (spp + 31u) / 32u;
+    return l;
+}
+
 // One path of pixel (px, py), sample `sample`.  kAdjoint = false: returns
 // the path radiance at emission scale 1 (the image multiplies by the scale).
 // kAdjoint = true: `total` is that radiance from the first replay; adds
@@ -136,10 +165,11 @@ WF_DEV void flush_vertex(uint32_t key, float4 value, float4* warp_buffer, const 
 // lanes without a path) and run the same number of vertex steps.
 // Tally: the traversal variant (Opaque<NoTally> for scenes that allow it,
 // wf_scene::opaque).
-template <bool kAdjoint, typename Tally>
+// kRecord: the non-adjoint replay fills `record`, the adjoint one reads it.
+template <bool kAdjoint, bool kRecord, typename Tally>
 WF_DEV V3 diff_path(const DeviceScene& s, const DiffParams& P, const DiffSettings& cfg, uint32_t px, uint32_t py,
                     uint32_t sample, bool alive, V3 total, V3 delta, const DiffGrads& G, float4* warp_buffer,
-                    uint32_t* error) {
+                    uint32_t* error, PathRecord* record) {
     V3 o{0.0f, 0.0f, 0.0f}, d{0.0f, 0.0f, 1.0f};
     uint64_t rng = 0;
     if (alive) {
@@ -159,7 +189,21 @@ WF_DEV V3 diff_path(const DeviceScene& s, const DiffParams& P, const DiffSetting
         do {
             if (!alive) break;
             alive = false;  // set again below when the path continues
-            TraceState h = trace_closest_call(s, o, d, tally);
+            TraceState h;
+            if (kAdjoint && depth < kReplayVertices) {
+                float4 r = record->hit[depth];
+                h.t = r.x;
+                h.u = r.y;
+                h.v = r.z;
+                h.prim = __float_as_uint(r.w);
+                h.inst = record->inst[depth];
+            } else {
+                h = trace_closest_call(s, o, d, tally);
+                if (kRecord && !kAdjoint && depth < kReplayVertices) {
+                    record->hit[depth] = make_float4(h.t, h.u, h.v, __uint_as_float(h.prim));
+                    record->inst[depth] = h.inst;
+                }
+            }
             SurfaceHit sh;
             if (!finish_hit(s, o, d, h.t, h.u, h.v, h.prim, h.inst, sh)) break;
             const Material& m = s.materials[sh.material];
@@ -200,7 +244,17 @@ WF_DEV V3 diff_path(const DeviceScene& s, const DiffParams& P, const DiffSetting
                     V3 st = offset_ray_origin(lp, light.normal, -wl, dist);
                     V3 seg = st - so;
                     float sd = length(seg);
-                    if (sd > kRayMinDistance && !trace_any_call(s, so, seg / sd, sd - kRayMinDistance, tally)) {
+                    bool visible = sd > kRayMinDistance;
+                    if (visible) {
+                        if (kAdjoint && depth < kReplayVertices) {
+                            visible = !(record->occluded >> depth & 1u);
+                        } else {
+                            visible = !trace_any_call(s, so, seg / sd, sd - kRayMinDistance, tally);
+                            if (kRecord && !kAdjoint && !visible && depth < kReplayVertices)
+                                record->occluded |= 1u << depth;
+                        }
+                    }
+                    if (visible) {
                         OrenNayar on = oren_nayar(n, wo, wl, sigma);
                         float geometry = cos_l * light.area / (dist2 * light.selection_pdf);
                         const Material& lm = s.materials[light.material];
@@ -244,20 +298,43 @@ WF_DEV V3 diff_path(const DeviceScene& s, const DiffParams& P, const DiffSetting
 
 // Both kernels trace one path per thread; bounded to 8 CTAs of 128 per SM
 // (64 registers) they keep enough warps resident to hide traversal latency.
-// Inverse-rendering config (512x512, 32 spp), with the opaque traversal:
-// forward 58.9 -> 42.0 ms, adjoint 182 -> 124.5 ms against the unbounded
-// kernels (138 and 168 registers, 3 CTAs per SM).
+// Image and gradients of the 256x256 inverse-rendering scene at 8 samples:
+// 26.9 ms with one pixel per thread (forward) and per warp (adjoint), 45.3 ms
+// with the wide BVHs alone (their node visits want full warps), 9.0 ms with
+// the lanes of DiffLanes and the replay record.
+//
+// The forward kernel takes one sample per lane, 32 / spp pixels to a warp
+// (DiffLanes): with one pixel per thread and its samples one after another, a
+// 256x256 image filled 512 of 1,184 resident CTAs.  The samples of a pixel
+// are added in sample order, as a serial loop adds them.
 template <typename Tally>
 __global__ void __launch_bounds__(128, 8) k_diff_forward(const __grid_constant__ DeviceScene s, DiffParams P,
                                                          DiffSettings cfg, float* image, uint32_t* error) {
     uint32_t n = cfg.w * cfg.h;
+    DiffLanes L = diff_lanes(cfg.spp);
+    uint32_t lane = threadIdx.x & 31;
+    uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    uint32_t groups = (n + L.pixels - 1) / L.pixels;
     DiffGrads none{};
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    for (uint32_t g = warp; g < groups; g += warps) {
+        uint32_t i = g * L.pixels + lane / L.samples;
+        bool owned = lane < L.pixels * L.samples && i < n;
         uint32_t px = cfg.x + i % cfg.w, py = cfg.y + i / cfg.w;
         V3 acc{0.0f, 0.0f, 0.0f};
-        for (uint32_t k = 0; k < cfg.spp; ++k)
-            acc += diff_path<false, Tally>(s, P, cfg, px, py, cfg.sample_start + k, true, V3{}, V3{}, none, nullptr,
-                                           error);
+        for (uint32_t chunk = 0; chunk < L.chunks; ++chunk) {
+            uint32_t k = chunk * 32 + lane % L.samples;
+            V3 u{0.0f, 0.0f, 0.0f};
+            if (owned && k < cfg.spp)
+                u = diff_path<false, false, Tally>(s, P, cfg, px, py, cfg.sample_start + k, true, V3{}, V3{}, none,
+                                                   nullptr, error, nullptr);
+            uint32_t first = lane - lane % L.samples;
+            uint32_t here = min(L.samples, cfg.spp - chunk * 32);
+            for (uint32_t j = 0; j < here; ++j)
+                acc += V3{__shfl_sync(0xffffffffu, u.x, int(first + j)), __shfl_sync(0xffffffffu, u.y, int(first + j)),
+                          __shfl_sync(0xffffffffu, u.z, int(first + j))};
+        }
+        if (!owned || lane % L.samples != 0) continue;
         float scale = P.emission_scale / float(cfg.spp);
         float* out = image + 3 * (size_t(py) * cfg.width + px);
         out[0] = acc.x * scale;
@@ -267,9 +344,10 @@ __global__ void __launch_bounds__(128, 8) k_diff_forward(const __grid_constant__
 }
 
 // d_image: dLoss/dImage (image = mean over samples of emission_scale * U).
-// Each warp takes up to 32 samples of one pixel, so the lanes of a warp
-// mostly hit the same triangles and their gradients merge before the
-// atomics (flush_vertex).
+// A warp takes the samples of one pixel, or of 32 / spp neighbouring pixels
+// (DiffLanes; 8 samples per pixel left 24 lanes idle), so its lanes mostly
+// hit the same triangles and their gradients merge before the atomics
+// (flush_vertex).
 template <typename Tally>
 __global__ void __launch_bounds__(128, 8) k_diff_backward(const __grid_constant__ DeviceScene s, DiffParams P,
                                                           DiffSettings cfg, const float* d_image, DiffGrads G,
@@ -279,24 +357,33 @@ __global__ void __launch_bounds__(128, 8) k_diff_backward(const __grid_constant_
     uint32_t lane = threadIdx.x & 31;
     uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    uint32_t chunks = (cfg.spp + 31) / 32;
-    uint32_t items = cfg.w * cfg.h * chunks;
+    DiffLanes L = diff_lanes(cfg.spp);
+    uint32_t n = cfg.w * cfg.h;
+    uint32_t items = (n + L.pixels - 1) / L.pixels * L.chunks;
     double d_scale = 0.0;
     DiffGrads none{};
+    PathRecord record;
     for (uint32_t item = warp; item < items; item += warps) {
-        uint32_t i = item / chunks, chunk = item % chunks;
+        uint32_t i = item / L.chunks * L.pixels + lane / L.samples;
+        uint32_t k = item % L.chunks * 32 + lane % L.samples;
+        bool alive = lane < L.pixels * L.samples && i < n && k < cfg.spp;
         uint32_t px = cfg.x + i % cfg.w, py = cfg.y + i / cfg.w;
-        const float* g = d_image + 3 * (size_t(py) * cfg.width + px);
-        V3 grad_pixel{g[0], g[1], g[2]};
-        if (grad_pixel.x == 0.0f && grad_pixel.y == 0.0f && grad_pixel.z == 0.0f) continue;  // uniform per warp
-        uint32_t k = chunk * 32 + lane;
-        bool alive = k < cfg.spp;
+        V3 grad_pixel{0.0f, 0.0f, 0.0f};
+        if (alive) {
+            const float* g = d_image + 3 * (size_t(py) * cfg.width + px);
+            grad_pixel = V3{g[0], g[1], g[2]};
+            alive = !(grad_pixel.x == 0.0f && grad_pixel.y == 0.0f && grad_pixel.z == 0.0f);
+        }
+        if (!__any_sync(0xffffffffu, alive)) continue;
         uint32_t sample = cfg.sample_start + k;
         // the image is scale/spp * sum U: dLoss/dU = dLoss/dImage * scale / spp
         V3 delta = grad_pixel * (P.emission_scale / float(cfg.spp));
         V3 total{0.0f, 0.0f, 0.0f};
-        if (alive) total = diff_path<false, Tally>(s, P, cfg, px, py, sample, true, V3{}, V3{}, none, nullptr, error);
-        diff_path<true, Tally>(s, P, cfg, px, py, sample, alive, total, delta, G, warp_buffer, error);
+        record.occluded = 0;
+        if (alive)
+            total = diff_path<false, true, Tally>(s, P, cfg, px, py, sample, true, V3{}, V3{}, none, nullptr, error,
+                                                  &record);
+        diff_path<true, true, Tally>(s, P, cfg, px, py, sample, alive, total, delta, G, warp_buffer, error, &record);
         if (alive) d_scale += double(dot(grad_pixel, total)) / double(cfg.spp);
     }
     for (int off = 16; off > 0; off >>= 1) d_scale += __shfl_down_sync(0xffffffffu, d_scale, off);
@@ -350,7 +437,12 @@ wf_status diff_finish(uint32_t* error, cudaStream_t st) {
     return WF_OK;
 }
 
-uint32_t diff_grid(uint32_t n) { return std::max(1u, std::min((n + 127) / 128, 148u * 16u)); }
+// Warps of four per block, one per DiffLanes item, up to two resident waves.
+uint32_t diff_grid(const DiffSettings& cfg) {
+    DiffLanes l = diff_lanes(cfg.spp);
+    uint64_t items = (uint64_t(cfg.w) * cfg.h + l.pixels - 1) / l.pixels * l.chunks;
+    return uint32_t(std::max<uint64_t>(1, std::min<uint64_t>((items + 3) / 4, 148u * 16u)));
+}
 
 }  // namespace
 }  // namespace wf
@@ -369,9 +461,9 @@ extern "C" wf_status wf_diff_forward(const wf_scene* scene, const wf_camera* cam
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync");
     DiffParams P{albedo, roughness, emission_scale};
     if (!scene->opaque())
-        k_diff_forward<NoTally><<<diff_grid(cfg.w * cfg.h), 128, 0, st>>>(scene->view, P, cfg, image, error);
+        k_diff_forward<NoTally><<<diff_grid(cfg), 128, 0, st>>>(scene->view, P, cfg, image, error);
     else
-        k_diff_forward<Opaque<NoTally>><<<diff_grid(cfg.w * cfg.h), 128, 0, st>>>(scene->view, P, cfg, image, error);
+        k_diff_forward<Opaque<NoTally>><<<diff_grid(cfg), 128, 0, st>>>(scene->view, P, cfg, image, error);
     ce = cudaGetLastError();
     if (ce != cudaSuccess) return cuda_fail(ce, "k_diff_forward");
     return diff_finish(error, st);
@@ -391,8 +483,7 @@ extern "C" wf_status wf_diff_backward(const wf_scene* scene, const wf_camera* ca
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync");
     DiffParams P{albedo, roughness, emission_scale};
     DiffGrads G{d_albedo, d_roughness, d_emission_scale};
-    uint32_t items = cfg.w * cfg.h * ((cfg.spp + 31) / 32);  // one warp each
-    uint32_t blocks = std::max(1u, std::min((items + 3) / 4, 148u * 16u));
+    uint32_t blocks = diff_grid(cfg);
     if (!scene->opaque())
         k_diff_backward<NoTally><<<blocks, 128, 0, st>>>(scene->view, P, cfg, d_image, G, error);
     else
