@@ -1,0 +1,61 @@
+"""Launches of every size through the trace and shadow kernels' ray feed.
+
+A launch of few rays uses some lanes of each warp, a larger one all of them
+and then refills.  Every path's radiance is independent of the launch it runs
+in, so a frame must not change with the number of samples per wave, the
+wavefronts per tile or the schedule (bit for bit), from one pixel to more rays
+than the launch has lanes."""
+import numpy as np
+import pytest
+
+import wfpt
+from wfpt import abi, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(which, w, h):
+    if which == "mesh":
+        return scenes.large_mesh(w, h, terrain_quads=48, instance_count=12, instance_frequency=8, glass_spheres=4,
+                                 env_size=(64, 32))
+    if which == "room":  # alpha-masked textures
+        return scenes.textured_room(w, h)
+    scene, cam = scenes.cornell_box(w, h)
+    if which == "lists":  # primitives outside the BVHs: the generic kernels
+        scene.static_triangles = scenes.quad((-1, 0, 1), (1, 0, 1), (1, 0.5, 1), (-1, 0.5, 1), 1)
+        scene.triangles = scenes.quad((-1, 1, 1), (0, 1, 1), (0, 2, 0.5), (-1, 2, 0.5), 2)
+    return scene, cam
+
+
+@pytest.mark.parametrize("which", ["cornell", "mesh", "room", "lists"])
+@pytest.mark.parametrize("size", [(1, 1), (3, 5), (65, 33), (257, 129)])
+def test_frame_does_not_depend_on_launch_size(cuda, which, size):
+    w, h = size
+    scene, cam = _scene(which, w, h)
+    dev = wfpt.DeviceScene(scene)
+    spp = 8
+    images = []
+    for fields in (dict(mode=abi.MODE_GRAPH), dict(mode=abi.MODE_GRAPH, samples_per_wave=8),
+                   dict(mode=abi.MODE_GRAPH, samples_per_wave=8, concurrent_tiles=1),
+                   dict(mode=abi.MODE_STREAM),
+                   dict(mode=abi.MODE_PERSISTENT, persistent_stages=abi.PERSISTENT_FUSED),
+                   dict(mode=abi.MODE_PERSISTENT, persistent_stages=abi.PERSISTENT_STAGED)):
+        r = wfpt.Renderer(dev, cam, wfpt.render_config(w, h, max_depth=8, rr_start_depth=4, **fields))
+        images.append(r.render_task((0, 0, w, h), 3, spp))
+        r.close()
+    dev.close()
+    for image in images[1:]:
+        assert np.array_equal(images[0].view(np.uint32), image.view(np.uint32))
+
+
+def test_more_rays_than_lanes(cuda):
+    """1.2 M rays per bounce against at most 151,552 lanes."""
+    scene, cam = scenes.cornell_box(320, 240)
+    dev = wfpt.DeviceScene(scene)
+    images = []
+    for wave in (1, 16):
+        r = wfpt.Renderer(dev, cam, wfpt.render_config(320, 240, max_depth=5, samples_per_wave=wave))
+        images.append(r.render_task((0, 0, 320, 240), 0, 16))
+        r.close()
+    dev.close()
+    assert np.array_equal(images[0].view(np.uint32), images[1].view(np.uint32))

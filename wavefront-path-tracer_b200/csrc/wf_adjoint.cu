@@ -92,8 +92,10 @@ WF_DEV V3 sample_cosine_hemisphere_uv(V3 n, float u1, float u2) {
     constexpr float two_pi = 6.28318530718f;
     float radius = sqrtf(u1);
     float phi = two_pi * u2;
-    float x = radius * wfm::cosf(phi);
-    float y = radius * wfm::sinf(phi);
+    float sin_phi, cos_phi;
+    wfm::sincosf(phi, sin_phi, cos_phi);
+    float x = radius * cos_phi;
+    float y = radius * sin_phi;
     float z = sqrtf(1.0f - u1);
     V3 helper = fabsf(n.x) > 0.1f ? V3{0.0f, 1.0f, 0.0f} : V3{1.0f, 0.0f, 0.0f};
     V3 tangent = normalize(cross(helper, n));

@@ -283,6 +283,7 @@ wf_status wf_scene_set_environment(wf_scene* s, const wf_environment* env) {
     up(&ev.probabilities, map.probabilities);
     up(&ev.alias, map.alias);
     up(&ev.row_solid_angle, map.row_solid_angle);
+    up(&ev.row_cosine, map.row_cosine);
     if (e != cudaSuccess) {
         free_list(s->env_allocations);
         ev = Environment{};

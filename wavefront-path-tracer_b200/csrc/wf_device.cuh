@@ -231,7 +231,8 @@ WF_HDI uint32_t material_category(const Material& mat) {
 struct TexBinding {
     uint32_t texture;  // kInvalid: none
     uint32_t texcoord;
-    float offset_x, offset_y, scale_x, scale_y, rotation;
+    float offset_x, offset_y, scale_x, scale_y;
+    float sine, cosine;  // of the rotation
     uint32_t has_transform;
 };
 
@@ -296,6 +297,7 @@ struct Environment {
     const float* probabilities;
     const float2* alias;           // (probability, alias index bits)
     const float* row_solid_angle;  // environmentSolidAngle(row), environment.cuh:35-39
+    const double* row_cosine;      // cos(pi k / height) of the height + 1 row edges
     uint32_t width, height;
     float intensity;
     float rotation;

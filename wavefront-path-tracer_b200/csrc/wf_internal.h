@@ -68,6 +68,7 @@ struct HostEnvironment {
     std::vector<float> probabilities;
     std::vector<float2> alias;
     std::vector<float> row_solid_angle;
+    std::vector<double> row_cosine;
     float intensity = 1.0f;
     float rotation = 0.0f;
 };

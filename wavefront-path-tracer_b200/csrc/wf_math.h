@@ -119,6 +119,24 @@ WF_HD_CALL double cos(double x) {
     }
 }
 
+// sin(x) and cos(x) of one reduction: the values of sin() and cos() above.
+WF_HD_CALL void sincos(double x, double& sine, double& cosine) {
+#if defined(WF_FAST_MATH) && defined(__CUDA_ARCH__)
+    ::sincos(x, &sine, &cosine);
+    return;
+#endif
+    if (!(x == x) || x == INFINITY || x == -INFINITY) {
+        sine = cosine = x - x;
+        return;
+    }
+    int q;
+    double r = reduce_pio2(x, q);
+    double a = sin_kernel(r), b = cos_kernel(r);
+    double s = (q & 1) ? b : a, c = (q & 1) ? a : b;
+    sine = (q & 2) ? -s : s;
+    cosine = ((q + 1) & 2) ? -c : c;
+}
+
 // atan(t) for 0 <= t <= 1: t > tan(15 deg) is folded by
 // atan(t) = pi/6 + atan((t*sqrt3 - 1) / (t + sqrt3)); the series
 // t - t^3/3 + t^5/5 - ... is summed through t^31.
@@ -254,6 +272,7 @@ WF_HD_CALL double pow(double x, double y) {
 // an image RMSE instead of bit for bit.
 WF_HD float sinf(float x) { return ::sinf(x); }
 WF_HD float cosf(float x) { return ::cosf(x); }
+WF_HD void sincosf(float x, float& s, float& c) { ::sincosf(x, &s, &c); }
 WF_HD float tanf(float x) { return ::tanf(x); }
 WF_HD float atan2f(float y, float x) { return ::atan2f(y, x); }
 WF_HD float logf(float x) { return ::logf(x); }
@@ -262,6 +281,12 @@ WF_HD float powf(float x, float y) { return ::powf(x, y); }
 #else
 WF_HD float sinf(float x) { return float(wfm::sin(double(x))); }
 WF_HD float cosf(float x) { return float(wfm::cos(double(x))); }
+WF_HD void sincosf(float x, float& s, float& c) {
+    double a, b;
+    wfm::sincos(double(x), a, b);
+    s = float(a);
+    c = float(b);
+}
 WF_HD float tanf(float x) {
     double d = double(x);
     return float(wfm::sin(d) / wfm::cos(d));

@@ -304,7 +304,7 @@ wf_status build_host_scene(const wf_scene_desc* d, HostScene& s) {
             for (uint32_t k = 0; k < kTexSlots; ++k) {
                 const wf_texture_binding& b = *slots[k];
                 mt.slot[k] = TexBinding{b.texture, b.texcoord, b.offset[0], b.offset[1], b.scale[0], b.scale[1],
-                                        b.rotation, b.has_transform};
+                                        wfm::sinf(b.rotation), wfm::cosf(b.rotation), b.has_transform};
                 any = any || b.texture < d->texture_count;
             }
             Material& m = s.materials.back();
@@ -613,6 +613,8 @@ wf_status build_environment(const wf_environment* env, HostEnvironment& map) {
     for (uint32_t i : large) map.alias[i] = make_float2(1.0f, bits_float(i));
     map.row_solid_angle.resize(h);
     for (uint32_t y = 0; y < h; ++y) map.row_solid_angle[y] = environment_solid_angle(y, w, h);
+    map.row_cosine.resize(size_t(h) + 1);
+    for (uint32_t y = 0; y <= h; ++y) map.row_cosine[y] = wfm::cos(3.14159265358979323846 * y / h);
     map.intensity = env->intensity;
     map.rotation = std::fmod(env->rotation_degrees, 360.0f) * (3.14159265359f / 180.0f);
     return WF_OK;

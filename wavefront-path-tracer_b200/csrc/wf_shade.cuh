@@ -96,8 +96,10 @@ WF_DEV V3 sample_cosine_hemisphere(V3 n, Path& path, uint32_t strategy) {
     float u2 = random_float(path.rng, strategy);
     float radius = sqrtf(u1);
     float phi = two_pi * u2;
-    float x = radius * wfm::cosf(phi);
-    float y = radius * wfm::sinf(phi);
+    float sin_phi, cos_phi;
+    wfm::sincosf(phi, sin_phi, cos_phi);
+    float x = radius * cos_phi;
+    float y = radius * sin_phi;
     float z = sqrtf(1.0f - u1);
     V3 helper = fabsf(n.x) > 0.1f ? V3{0.0f, 1.0f, 0.0f} : V3{1.0f, 0.0f, 0.0f};
     V3 tangent = normalize(cross(helper, n));
@@ -212,15 +214,17 @@ WF_DEV V3 sg_basis(V3 n, float x, float y, float z) {
 }
 WF_DEV V3 sg_sample(const SpecGloss& s, V3 n, V3 outgoing, float choice, float u, float v) {
     float phi = 6.28318530718f * v;
+    float sin_phi, cos_phi;
+    wfm::sincosf(phi, sin_phi, cos_phi);
     if (choice < sg_probability(s)) {
         float alpha = sg_alpha(s);
         float cosine = sqrtf((1.0f - u) / (1.0f + (alpha * alpha - 1.0f) * u));
         float sine = sqrtf(fmaxf(0.0f, 1.0f - cosine * cosine));
-        V3 half = sg_basis(n, sine * wfm::cosf(phi), sine * wfm::sinf(phi), cosine);
+        V3 half = sg_basis(n, sine * cos_phi, sine * sin_phi, cosine);
         return 2.0f * dot(outgoing, half) * half - outgoing;
     }
     float radius = sqrtf(u);
-    return sg_basis(n, radius * wfm::cosf(phi), radius * wfm::sinf(phi), sqrtf(1.0f - u));
+    return sg_basis(n, radius * cos_phi, radius * sin_phi, sqrtf(1.0f - u));
 }
 
 // include/renderer/gltf_pbr.cuh:8-119.
@@ -298,7 +302,9 @@ WF_DEV V3 pbr_sample_reflection(V3 normal, V3 view, float roughness, float u, fl
     float alpha = pbr_alpha(roughness);
     float cosine = sqrtf((1.f - u) / ((1.f - u) + alpha * alpha * u));
     float sine = sqrtf(fmaxf(0.f, 1.f - cosine * cosine)), phi = 6.28318530718f * v;
-    V3 half = sg_basis(normal, sine * wfm::cosf(phi), sine * wfm::sinf(phi), cosine);
+    float sin_phi, cos_phi;
+    wfm::sincosf(phi, sin_phi, cos_phi);
+    V3 half = sg_basis(normal, sine * cos_phi, sine * sin_phi, cosine);
     return 2.f * dot(view, half) * half - view;
 }
 WF_CALL V3 pbr_evaluate_cos(const GltfPbr& s, V3 view, V3 light, float diffuse_pdf, float& pdf) {
@@ -325,21 +331,33 @@ WF_CALL V3 pbr_evaluate_cos(const GltfPbr& s, V3 view, V3 light, float diffuse_p
 WF_DEV V3 rotate_env(V3 d, float c, float s) {
     return V3{c * d.x + s * d.z, d.y, -s * d.x + c * d.z};
 }
-WF_DEV void environment_uv(const Environment& e, V3 world, float& u, float& v) {
-    V3 d = rotate_env(world, e.cos_neg, e.sin_neg);
-    u = wfm::atan2f(d.z, d.x) / (2.0f * kPiF) + 0.5f;
-    u -= floorf(u);
-    float vv = wfm::atan2f(sqrtf(d.x * d.x + d.z * d.z), d.y) / kPiF;
-    v = fminf(1.0f, fmaxf(0.0f, vv));
-}
-WF_CALL float environment_pdf(const Environment& e, V3 direction) {
-    if (e.width == 0 || e.height == 0 || e.probabilities == nullptr) return 0.0f;
+// Map coordinates of a direction: two double-precision arctangents, the
+// dearest part of a lookup, so a direction whose density and radiance are
+// both wanted is mapped once.
+struct EnvUv {
     float u, v;
-    environment_uv(e, direction, u, v);
-    uint32_t x = uint32_t(u * e.width);
-    uint32_t y = uint32_t(v * e.height);
-    uint32_t index = (y < e.height ? y : e.height - 1) * e.width + (x < e.width ? x : e.width - 1);
-    return e.probabilities[index] / e.row_solid_angle[index / e.width];
+};
+WF_CALL EnvUv environment_uv(const Environment& e, V3 world) {
+    V3 d = rotate_env(world, e.cos_neg, e.sin_neg);
+    EnvUv r;
+    r.u = wfm::atan2f(d.z, d.x) / (2.0f * kPiF) + 0.5f;
+    r.u -= floorf(r.u);
+    float vv = wfm::atan2f(sqrtf(d.x * d.x + d.z * d.z), d.y) / kPiF;
+    r.v = fminf(1.0f, fmaxf(0.0f, vv));
+    return r;
+}
+WF_DEV bool environment_empty(const Environment& e) {
+    return e.width == 0 || e.height == 0 || e.probabilities == nullptr;
+}
+WF_DEV float environment_pdf(const Environment& e, EnvUv at) {
+    if (environment_empty(e)) return 0.0f;
+    uint32_t x = min(uint32_t(at.u * e.width), e.width - 1);
+    uint32_t y = min(uint32_t(at.v * e.height), e.height - 1);
+    return e.probabilities[size_t(y) * e.width + x] / e.row_solid_angle[y];
+}
+WF_DEV float environment_pdf(const Environment& e, V3 direction) {
+    if (environment_empty(e)) return 0.0f;
+    return environment_pdf(e, environment_uv(e, direction));
 }
 // Bilinear lookup: normalized coordinates, wrap in u, clamp in v, weights
 // (1-f, f), rows then columns (the texture of scene.cu:318-328 with the
@@ -352,7 +370,8 @@ WF_CALL V3 environment_texel(const Environment& e, float u, float v) {
     int w = int(e.width), h = int(e.height);
     for (int j = 0; j < 2; ++j)
         for (int i = 0; i < 2; ++i) {
-            int xx = ((x + i) % w + w) % w;
+            int xx = x + i;  // -1 to w: u is in [0, 1]
+            xx = xx < 0 ? xx + w : xx >= w ? xx - w : xx;
             int yy = min(max(y + j, 0), h - 1);
             float4 p = __ldg(&e.pixels[size_t(yy) * e.width + xx]);
             float wt = (i ? fx : 1 - fx) * (j ? fy : 1 - fy);
@@ -362,10 +381,9 @@ WF_CALL V3 environment_texel(const Environment& e, float u, float v) {
         }
     return V3{rx, ry, rz};
 }
-WF_CALL V3 environment_radiance(const Environment& e, V3 direction) {
-    float u, v;
-    environment_uv(e, direction, u, v);
-    return environment_texel(e, u, v) * e.intensity;
+WF_DEV V3 environment_radiance(const Environment& e, EnvUv at) { return environment_texel(e, at.u, at.v) * e.intensity; }
+WF_DEV V3 environment_radiance(const Environment& e, V3 direction) {
+    return environment_radiance(e, environment_uv(e, direction));
 }
 struct EnvSample {
     V3 direction;
@@ -382,10 +400,12 @@ WF_CALL EnvSample sample_environment(const Environment& e, double candidate, flo
     uint32_t x = index % e.width, y = index / e.width;
     double u = (x + fminf(1.0f - 1.0e-7f, fmaxf(1.0e-7f, longitude))) / e.width;
     double jitter = fminf(1.0f - 1.0e-7f, fmaxf(1.0e-7f, latitude));
-    double cosine = (1.0 - jitter) * wfm::cos(pi * y / e.height) + jitter * wfm::cos(pi * (y + 1.0) / e.height);
+    double cosine = (1.0 - jitter) * __ldg(&e.row_cosine[y]) + jitter * __ldg(&e.row_cosine[y + 1]);
     double sine = sqrt(fmax(0.0, 1.0 - cosine * cosine));
     double phi = (u - 0.5) * 2 * pi;
-    V3 local{float(sine * wfm::cos(phi)), float(cosine), float(sine * wfm::sin(phi))};
+    double sin_phi, cos_phi;
+    wfm::sincos(phi, sin_phi, cos_phi);
+    V3 local{float(sine * cos_phi), float(cosine), float(sine * sin_phi)};
     return EnvSample{rotate_env(local, e.cos_rot, e.sin_rot), e.probabilities[index] / e.row_solid_angle[y]};
 }
 
@@ -396,11 +416,13 @@ WF_DEV float power_heuristic(float a, float b) {
     return a2 / (a2 + b2);
 }
 
-WF_DEV float diffuse_continuation_pdf(const DeviceScene& s, V3 normal, V3 direction) {
+// `at`: the direction's map coordinates where the caller has them, or null.
+WF_DEV float diffuse_continuation_pdf(const DeviceScene& s, V3 normal, V3 direction, const EnvUv* at = nullptr) {
     float probability = s.env.sampling ? 0.5f : 0.0f;
     float cosine_pdf = fmaxf(0.0f, dot(normal, direction)) * 0.31830988618f;
-    return probability > 0.0f ? (1.0f - probability) * cosine_pdf + probability * environment_pdf(s.env, direction)
-                              : cosine_pdf;
+    if (!(probability > 0.0f)) return cosine_pdf;
+    float environment = at ? environment_pdf(s.env, *at) : environment_pdf(s.env, direction);
+    return (1.0f - probability) * cosine_pdf + probability * environment;
 }
 
 WF_DEV EnvSample sample_path_environment(const DeviceScene& s, Path& path, uint32_t strategy) {
@@ -514,8 +536,11 @@ WF_CALL V3 material_normal(const DeviceScene& s, const TexBinding& b, float norm
 }
 
 // evaluateSurface, device_traversal.cuh:427-441.
+// `at`: incoming's environment map coordinates where the caller has them
+// (at.u >= 0).
+constexpr EnvUv kNoUv{-1.0f, 0.0f};
 WF_CALL V3 evaluate_surface(const DeviceScene& s, const Material& m, const ShadeHit& hit, V3 outgoing, V3 incoming,
-                           float& pdf) {
+                           EnvUv at, float& pdf) {
     if (m.type == kSpecGloss)
         return sg_evaluate(SpecGloss{m.albedo, m.specular, material_roughness(m)}, hit.normal, outgoing, incoming, pdf);
     uint32_t effective = m.type == kDiffuse && m.metallic > 0.5f ? uint32_t(kMetal) : m.type;
@@ -526,7 +551,7 @@ WF_CALL V3 evaluate_surface(const DeviceScene& s, const Material& m, const Shade
         }
         return sg_evaluate(SpecGloss{V3{0, 0, 0}, m.albedo, material_roughness(m)}, hit.normal, outgoing, incoming, pdf);
     }
-    pdf = diffuse_continuation_pdf(s, hit.normal, incoming);
+    pdf = diffuse_continuation_pdf(s, hit.normal, incoming, at.u >= 0.0f ? &at : nullptr);
     return m.albedo * 0.31830988618f;
 }
 
@@ -556,13 +581,14 @@ WF_CALL GltfPbr gltf_surface(const Material& m, const ShadeHit& hit, const Shade
 
 // evaluateSurfaceCos, device_traversal.cuh:519-527.
 WF_CALL V3 evaluate_surface_cos(const DeviceScene& s, const Material& m, const ShadeHit& hit, const ShadeHit& shaded,
-                               V3 view, V3 light, float& pdf) {
+                               V3 view, V3 light, EnvUv at, float& pdf) {
     if (m.flags & kMatGltfPbr) {
         GltfPbr g = gltf_surface(m, hit, shaded);
         correct_gltf_normals(g, hit.geometric_normal, view);
-        return pbr_evaluate_cos(g, view, light, diffuse_continuation_pdf(s, g.normal, light), pdf);
+        return pbr_evaluate_cos(
+            g, view, light, diffuse_continuation_pdf(s, g.normal, light, at.u >= 0.0f ? &at : nullptr), pdf);
     }
-    return evaluate_surface(s, m, shaded, view, light, pdf) * fmaxf(0.f, dot(shaded.normal, light));
+    return evaluate_surface(s, m, shaded, view, light, at, pdf) * fmaxf(0.f, dot(shaded.normal, light));
 }
 
 // ------------------------------------------------------------------ sinks
@@ -700,7 +726,7 @@ WF_DEV void sample_direct_light(const DeviceScene& s, const RenderParams& rp, Pa
     float geometry_term = light_cosine * light.area / (distance_squared * light.selection_pdf);
     float light_pdf = light.selection_pdf * distance_squared / (light_cosine * light.area);
     float bsdf_pdf;
-    V3 bsdf = evaluate_surface_cos(s, m, hit, shaded, -path.direction, direction, bsdf_pdf);
+    V3 bsdf = evaluate_surface_cos(s, m, hit, shaded, -path.direction, direction, kNoUv, bsdf_pdf);
     float mis = power_heuristic(light_pdf, bsdf_pdf);
     V3 direct = hadamard(bsdf, lm.emission) * (geometry_term * mis);
     sink.term(clamp_contribution(path, hadamard(path.throughput, direct), rp.clamp, false), handle);
@@ -765,7 +791,7 @@ WF_DEV void add_punctual_light(const DeviceScene& s, const RenderParams& rp, Pat
     if (!s.ignore_direct_light_occlusion) handle = sink.request(origin, direction, shadow_distance - kRayMinDistance);
     if (!sink.may_be_visible(handle)) return;
     float ignored;
-    V3 bsdf = evaluate_surface_cos(s, m, hit, shaded, -path.direction, light.direction, ignored);
+    V3 bsdf = evaluate_surface_cos(s, m, hit, shaded, -path.direction, light.direction, kNoUv, ignored);
     V3 direct = hadamard(bsdf, light.incident) * inverse_selection_pdf;
     sink.term(clamp_contribution(path, hadamard(path.throughput, direct), rp.clamp, false), handle);
 }
@@ -797,9 +823,10 @@ WF_DEV void sample_direct_environment(const DeviceScene& s, const RenderParams& 
     if (!s.ignore_direct_light_occlusion) handle = sink.request(origin, light.direction, 1.0e30f);
     if (!sink.may_be_visible(handle)) return;
     float bsdf_pdf;
-    V3 bsdf = evaluate_surface_cos(s, m, hit, shaded, -path.direction, light.direction, bsdf_pdf);
+    EnvUv at = environment_uv(e, light.direction);
+    V3 bsdf = evaluate_surface_cos(s, m, hit, shaded, -path.direction, light.direction, at, bsdf_pdf);
     float weight = power_heuristic(light.pdf, bsdf_pdf);
-    V3 direct = hadamard(bsdf, environment_radiance(e, light.direction)) * (weight / light.pdf);
+    V3 direct = hadamard(bsdf, environment_radiance(e, at)) * (weight / light.pdf);
     sink.term(clamp_contribution(path, hadamard(path.throughput, direct), rp.clamp, false), handle);
 }
 
@@ -807,10 +834,10 @@ WF_DEV void sample_direct_environment(const DeviceScene& s, const RenderParams& 
 template <typename Sink>
 WF_DEV void add_environment_or_sky(const DeviceScene& s, const RenderParams& rp, const Path& path, Sink& sink) {
     if (s.env.present) {
-        float weight = path.depth > 0 && !path.specular
-                           ? power_heuristic(path.prev_pdf, environment_pdf(s.env, path.direction))
-                           : 1.0f;
-        V3 c = hadamard(path.throughput, environment_radiance(s.env, path.direction)) * weight;
+        EnvUv at = environment_uv(s.env, path.direction);
+        float weight =
+            path.depth > 0 && !path.specular ? power_heuristic(path.prev_pdf, environment_pdf(s.env, at)) : 1.0f;
+        V3 c = hadamard(path.throughput, environment_radiance(s.env, at)) * weight;
         sink.term(clamp_contribution(path, c, rp.clamp, true), kUnconditional);
     } else if (!s.black_background) {
         float t = 0.5f * (path.direction.y + 1.0f);
@@ -1142,11 +1169,12 @@ WF_DEV V3 continue_diffuse(const DeviceScene& s, const RenderParams& rp, Path& p
                        ? sample_path_environment(s, path, rp.rng).direction
                        : sample_cosine_hemisphere(shaded.normal, path, rp.rng);
     float cosine = dot(shaded.normal, direction);
+    // half the environment's samples end here: before the density's lookup
+    path.active = !(cosine <= 0.0f || dot(direction, hit.geometric_normal) <= 0.0f);
+    if (!path.active) return direction;
     float pdf = diffuse_continuation_pdf(s, shaded.normal, direction);
-    if (!(pdf > 0.0f) || cosine <= 0.0f || dot(direction, hit.geometric_normal) <= 0.0f) {
-        path.active = false;
-        return direction;
-    }
+    path.active = pdf > 0.0f;
+    if (!path.active) return direction;
     path.throughput = hadamard(path.throughput, m.albedo) * (cosine * 0.31830988618f / pdf);
     path.prev_pdf = pdf;
     path.specular = false;

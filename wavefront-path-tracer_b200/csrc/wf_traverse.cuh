@@ -157,9 +157,15 @@ WF_DEV float4 texture_fetch(const DeviceScene& s, uint32_t texture, float u, flo
     float fx = tx - float(x), fy = ty - float(y);
     const float scale = 1.0f / 255.0f;
     float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    // wrapped texel columns and rows: one remainder per axis (the neighbour
+    // follows from it) instead of four per texel
+    int x0 = x % w, y0 = y % h;
+    if (x0 < 0) x0 += w;
+    if (y0 < 0) y0 += h;
+    int x1 = x0 + 1 == w ? 0 : x0 + 1, y1 = y0 + 1 == h ? 0 : y0 + 1;
     for (int j = 0; j < 2; ++j)
         for (int i = 0; i < 2; ++i) {
-            int xx = (((x + i) % w) + w) % w, yy = (((y + j) % h) + h) % h;
+            int xx = i ? x1 : x0, yy = j ? y1 : y0;
             uchar4 p = s.texels[info.z + size_t(yy) * uint32_t(w) + uint32_t(xx)];
             float wt = (i ? fx : 1.0f - fx) * (j ? fy : 1.0f - fy);
             r.x += wt * (float(p.x) * scale);
@@ -190,8 +196,7 @@ WF_DEV float4 sample_binding(const DeviceScene& s, const TexBinding& b, float2 u
     if (b.has_transform) {
         t.x *= b.scale_x;
         t.y *= b.scale_y;
-        float sine = wfm::sinf(b.rotation), cosine = wfm::cosf(b.rotation);
-        t = make_float2(cosine * t.x - sine * t.y + b.offset_x, sine * t.x + cosine * t.y + b.offset_y);
+        t = make_float2(b.cosine * t.x - b.sine * t.y + b.offset_x, b.sine * t.x + b.cosine * t.y + b.offset_y);
     }
     return texture_fetch(s, b.texture, t.x, 1.0f - t.y);
 }

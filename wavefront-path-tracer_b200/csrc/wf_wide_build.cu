@@ -59,13 +59,16 @@ cudaError_t build_wide_bvh(DeviceScene& view, const std::vector<BvhRef>& roots, 
     uint32_t root_count = uint32_t(roots.size());
     // Wide nodes other than the roots stand for distinct internal BVH2 nodes.
     size_t capacity = size_t(node_count) + root_count;
-    uint32_t *items = nullptr, *counters = nullptr;
-    uint2* bases = nullptr;
-    BvhRef* root_refs = nullptr;
-    cudaError_t e = device_alloc(reinterpret_cast<void**>(&items), capacity * sizeof(uint32_t));
-    if (e == cudaSuccess) e = device_alloc(reinterpret_cast<void**>(&bases), capacity * sizeof(uint2));
-    if (e == cudaSuccess) e = device_alloc(reinterpret_cast<void**>(&counters), 4 * sizeof(uint32_t));
-    if (e == cudaSuccess) e = device_alloc(reinterpret_cast<void**>(&root_refs), root_count * sizeof(BvhRef));
+    // one allocation: counters, bases, items, root refs (each part's alignment
+    // divides the size of those before it)
+    static_assert(sizeof(BvhRef) % sizeof(uint32_t) == 0 && alignof(BvhRef) == sizeof(uint32_t), "packed after words");
+    char* scratch = nullptr;
+    cudaError_t e = device_alloc(reinterpret_cast<void**>(&scratch),
+                                 16 + capacity * (sizeof(uint2) + sizeof(uint32_t)) + root_count * sizeof(BvhRef));
+    uint32_t* counters = reinterpret_cast<uint32_t*>(scratch);
+    uint2* bases = reinterpret_cast<uint2*>(scratch + 16);
+    uint32_t* items = reinterpret_cast<uint32_t*>(bases + capacity);
+    BvhRef* root_refs = reinterpret_cast<BvhRef*>(items + capacity);
     uint32_t host[4] = {root_count, 0, 0, 0};
     if (e == cudaSuccess) {
         std::vector<uint32_t> first(root_count);
@@ -105,10 +108,7 @@ cudaError_t build_wide_bvh(DeviceScene& view, const std::vector<BvhRef>& roots, 
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    cudaFree(items);
-    cudaFree(bases);
-    cudaFree(counters);
-    cudaFree(root_refs);
+    cudaFree(scratch);
     if (e == cudaSuccess) view.wide = WideBvh{nodes, triangles, leaves, host[3] ? 0u : 1u};
     return e;
 }
