@@ -157,6 +157,7 @@ wf_status wf_scene_create(const wf_scene_desc* desc, wf_scene** out) {
     if (wf_status e = build_host_scene(desc, h)) return e;
     auto s = std::make_unique<wf_scene>();
     WF_CUDA(cudaGetDevice(&s->device));
+    WF_CUDA(cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, s->device));
     DeviceScene& v = s->view;
     auto& L = s->allocations;
     uint64_t& B = s->device_bytes;

@@ -106,4 +106,5 @@ struct wf_scene {
     uint32_t material_categories = 0;  // bit k: some material has shading category k (material_category)
     wf::Box bounds{};
     int device = 0;
+    int sm_count = 148;
 };
