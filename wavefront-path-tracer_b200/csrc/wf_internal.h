@@ -97,11 +97,13 @@ struct wf_scene {
     uint32_t gpu_bvh_builds = 0;
     double bvh_build_ms = 0.0;
     bool alpha_textures = false;  // some material is alpha-masked with an albedo texture
-    // neither alpha-textured materials nor primitives outside the BVHs: the Opaque<> kernels
-    bool opaque() const {
-        return !alpha_textures && view.direct_instance_count == 0 && view.static_count == 0 &&
+    // every primitive is in a BVH (direct spheres aside): the Listless<> kernels
+    bool listless() const {
+        return view.direct_instance_count == 0 && view.static_count == 0 &&
                (view.direct_count == 0 || view.direct_bvh.root != wf::kNoRoot);
     }
+    // ... and no material is alpha-textured: the Opaque<> kernels
+    bool opaque() const { return !alpha_textures && listless(); }
     bool textured = false;        // some material has a texture binding
     uint32_t material_categories = 0;  // bit k: some material has shading category k (material_category)
     wf::Box bounds{};

@@ -95,6 +95,7 @@ struct wf_renderer {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     bool opaque = true;     // wf_scene::opaque: the Opaque<> trace and shadow kernels
+    bool listless = true;   // wf_scene::listless: the Listless<> ones otherwise
     bool textured = false;  // some textured material: k_shade<true>
     bool sort_shading = true;  // material-sort the hits before shading (k_classify, k_scatter)
     int device = 0;

@@ -54,6 +54,11 @@ struct Opaque : Base {
     static constexpr bool kAlphaTextures = false;
     static constexpr bool kLinearLists = false;
 };
+// Alpha-textured materials, but every primitive in a BVH (wf_scene::listless).
+template <typename Base>
+struct Listless : Base {
+    static constexpr bool kLinearLists = false;
+};
 
 struct TraceState {
     float t;          // closestT
