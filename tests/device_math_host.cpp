@@ -31,3 +31,12 @@ extern "C" void fetch_texture(const unsigned char* rgba, uint32_t w, uint32_t h,
         std::memcpy(out + 4 * i, &r, 16);
     }
 }
+
+// tile_pixel of every k of a w x h tile.
+extern "C" void tile_pixels(uint32_t w, uint32_t h, uint32_t* xy) {
+    for (uint32_t k = 0; k < w * h; ++k) {
+        uint2 at = tile_pixel(k, w, h);
+        xy[2 * k] = at.x;
+        xy[2 * k + 1] = at.y;
+    }
+}

@@ -1,6 +1,7 @@
 """Shading helpers on the CPU (a host build of the device headers): sincos()
-gives the bits of sin() and cos(), and the texture fetch wraps its texels as
-the remainder of each texel's coordinates does."""
+gives the bits of sin() and cos(), the texture fetch wraps its texels as the
+remainder of each texel's coordinates does, and the tile order names every
+pixel once."""
 import ctypes as C
 import shutil
 import subprocess
@@ -59,3 +60,15 @@ def test_texture_fetch_wraps(lib, size):
             p = texels[(y + j) % h, (x + i) % w].astype(f) * f(1.0 / 255.0)
             want += weight[:, None] * p
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("size", [(1, 1), (7, 3), (8, 4), (9, 5), (3, 40), (40, 3), (64, 32), (65, 33), (250, 131)])
+def test_tile_order_names_every_pixel_once(lib, size):
+    w, h = size
+    xy = np.zeros((w * h, 2), np.uint32)
+    lib.tile_pixels(C.c_uint32(w), C.c_uint32(h), C.c_void_p(xy.ctypes.data))
+    assert (xy[:, 0] < w).all() and (xy[:, 1] < h).all()
+    assert len(np.unique(xy[:, 1].astype(np.int64) * w + xy[:, 0])) == w * h
+    for k in range(0, (w // 8 * 8) * (h // 4 * 4), 32):  # whole blocks are 8 x 4
+        block = xy[k:k + 32]
+        assert (np.ptp(block, axis=0) == (7, 3)).all() and (block[0] % (8, 4) == 0).all()

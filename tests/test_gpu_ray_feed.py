@@ -59,3 +59,26 @@ def test_more_rays_than_lanes(cuda):
         r.close()
     dev.close()
     assert np.array_equal(images[0].view(np.uint32), images[1].view(np.uint32))
+
+
+@pytest.mark.parametrize("which", ["mesh", "room", "lists"])
+def test_large_ray_batches_match_small_ones(cuda, which):
+    """Batches around the size from which lanes are refilled (8 CTAs of 128 on
+    each SM, twice) against the same rays in small ones, record for record."""
+    scene, _ = _scene(which, 64, 36)
+    dev = wfpt.DeviceScene(scene)
+    line = cuda.cuda.get_device_properties(0).multi_processor_count * 8 * 256
+    rng = np.random.default_rng(2)
+    rays = np.zeros(line + 4097, abi.RAY_DTYPE)
+    rays["origin"] = rng.uniform(-2, 3, (len(rays), 3))
+    d = rng.normal(0, 1, (len(rays), 3))
+    rays["direction"] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    rays["direction"][::1001] *= np.float32(1e-8)  # past the wide test's bounds: the BVH2s decide
+    limit = rng.uniform(0.1, 6.0, len(rays)).astype(np.float32)
+    part = 50_000
+    hits = np.concatenate([dev.trace_closest(rays[k:k + part]) for k in range(0, len(rays), part)])
+    occluded = np.concatenate([dev.trace_any(rays[k:k + part], limit[k:k + part]) for k in range(0, len(rays), part)])
+    for count in (line - 1, line, line + 1, len(rays)):
+        assert dev.trace_closest(rays[:count]).tobytes() == hits[:count].tobytes()
+        assert np.array_equal(dev.trace_any(rays[:count], limit[:count]), occluded[:count])
+    dev.close()

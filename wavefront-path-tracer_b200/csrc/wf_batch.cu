@@ -2,7 +2,7 @@
 // sample range) in one captured CUDA graph.
 //
 // Work is a list of path units, one per (job, sample, pixel), job by job
-// and, within a job, sample by sample in pixel order.  A pool of path slots
+// and, within a job, sample by sample in the order of tile_pixel.  A pool of path slots
 // runs the wavefront stages of the single-scene renderer (lane-refill
 // closest hit, shading with deferred shadow rays, lane-refill occlusion,
 // ordered term accumulation and compaction) inside a device-side WHILE
@@ -146,7 +146,8 @@ __global__ void k_batch_accumulate(BatchView b, const Counters* c) {
         uint32_t q = t - b.order_pixels[pos];
         uint64_t first = J.unit_begin, last = first + uint64_t(J.pixels) * J.sample_count;
         if (last <= begin || first >= end) continue;
-        float* f = b.framebuffer + J.fb_offset + 3 * size_t(q);
+        uint2 at = tile_pixel(q, J.rp.width, J.rp.height);
+        float* f = b.framebuffer + J.fb_offset + 3 * (size_t(at.y) * J.rp.width + at.x);
         float r = f[0], g = f[1], bl = f[2];
         for (uint32_t k = 0; k < J.sample_count; ++k) {
             uint64_t unit = first + uint64_t(k) * J.pixels + q;

@@ -359,6 +359,26 @@ struct DeviceScene {
     float normal_map_min_cosine;
 };
 
+// ---------------------------------------------------------------- pixels
+// Pixel k of a w x h tile: blocks of 8 x 4 pixels one after another, so that
+// the 32 lanes of a warp see a compact patch of the image (camera rays visit
+// fewer different nodes than along a row of 32: 1080p guides 2.92 -> 2.32 ms,
+// the 1080p mesh 64.5 -> 62.0 ms), then the columns to the right of the last
+// whole block, then the rows below.
+WF_HDI uint2 tile_pixel(uint32_t k, uint32_t w, uint32_t h) {
+    uint32_t across = w >> 3, whole = (across << 3) * (h & ~3u);
+    if (k < whole) {
+        uint32_t block = k >> 5, in = k & 31u;
+        uint32_t row = block / across;
+        return make_uint2((block - row * across) * 8u + (in & 7u), row * 4u + (in >> 3));
+    }
+    k -= whole;
+    uint32_t rest = w & 7u, right = rest * (h & ~3u);
+    if (k < right) return make_uint2((across << 3) + k % rest, k / rest);
+    k -= right;
+    return make_uint2(k % w, (h & ~3u) + k / w);
+}
+
 // ----------------------------------------------------------- parameters
 struct Camera {
     V3 position, forward, right, up;

@@ -12,7 +12,7 @@
 // 56-byte store per pixel, so it is bound by traversal latency like the
 // renderer's trace kernels, and resident warps are what hide it.
 #include "wf_renderer.h"
-#include "wf_shade.cuh"
+#include "wf_wavefront.cuh"
 
 #define WF_CUDA(call)                                          \
     do {                                                       \
@@ -60,10 +60,11 @@ WF_DEV bool closest_surface(const DeviceScene& s, V3 o, V3 d, SurfaceHit& sh) {
 __global__ void __launch_bounds__(128, 8) k_frame_guides(const __grid_constant__ DeviceScene s, Camera camera,
                                                       Camera previous, uint32_t has_previous, uint32_t width,
                                                       uint32_t height, uint32_t x0, uint32_t y0, uint32_t tile_w,
-                                                      uint32_t count, wf_frame_guide* out) {
-    uint32_t index = blockIdx.x * blockDim.x + threadIdx.x;
-    if (index >= count) return;
-    uint32_t x = x0 + index % tile_w, y = y0 + index / tile_w;
+                                                      uint32_t tile_h, wf_frame_guide* out) {
+    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= tile_w * tile_h) return;
+    uint2 at = tile_pixel(k, tile_w, tile_h);
+    uint32_t x = x0 + at.x, y = y0 + at.y, index = at.y * tile_w + at.x;
     V3 o, d;
     camera_ray(camera, (x + 0.5f) / width, (y + 0.5f) / height, o, d);
     wf_frame_guide g;
@@ -130,8 +131,8 @@ wf_status frame_guides(const wf_scene* scene, const wf_camera* camera, const wf_
     Camera now = device_camera(*camera);
     Camera before = previous ? device_camera(*previous) : now;
     uint32_t blocks = uint32_t((count + 127) / 128);
-    k_frame_guides<<<blocks, 128, 0, stream>>>(scene->view, now, before, previous ? 1u : 0u, width, height, x, y, w,
-                                              uint32_t(count), guides);
+    k_frame_guides<<<blocks, 128, 0, stream>>>(scene->view, now, before, previous ? 1u : 0u, width, height, x, y, w, h,
+                                              guides);
     WF_CUDA(cudaGetLastError());
     return WF_OK;
 }

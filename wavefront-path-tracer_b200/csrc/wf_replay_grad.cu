@@ -90,7 +90,8 @@ __global__ void __launch_bounds__(128, 8) k_albedo_gradient(const __grid_constan
     for (uint32_t m = 0; m < kGradMaterials; ++m) grad[m] = V3{0.0f, 0.0f, 0.0f};
     uint32_t pixels = tile.width * tile.height;
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < pixels; q += gridDim.x * blockDim.x) {
-        uint32_t pixel = (tile.y + q / tile.width) * rp.width + tile.x + q % tile.width;
+        uint2 at = tile_pixel(q, tile.width, tile.height);
+        uint32_t pixel = (tile.y + at.y) * rp.width + tile.x + at.x;
         V3 adj{adjoint[3 * size_t(pixel)], adjoint[3 * size_t(pixel) + 1], adjoint[3 * size_t(pixel) + 2]};
         float sum_r = 0.0f, sum_g = 0.0f, sum_b = 0.0f;  // the cleared tile, then each sample in order
         for (uint32_t k = 0; k < samples; ++k) {

@@ -42,8 +42,9 @@ WF_DEV void store_path(const PathSoA& ps, uint32_t p, const Path& path) {
 
 // generatePrimaryRays, src/renderer/renderer.cu:10-42.
 WF_DEV void init_path(const RenderParams& rp, const TileDev& tile, uint32_t sample, uint32_t lp, Path& path) {
-    uint32_t x = tile.x + lp % tile.width;
-    uint32_t y = tile.y + lp / tile.width;
+    uint2 at = tile_pixel(lp, tile.width, tile.height);
+    uint32_t x = tile.x + at.x;
+    uint32_t y = tile.y + at.y;
     uint32_t pixel = y * rp.width + x;
     uint64_t rng = make_rng_state(pixel_rng_key(pixel, sample, rp.rng), rp.rng);
     float u = (float(x) + random_float(rng, rp.rng)) / float(rp.width);
