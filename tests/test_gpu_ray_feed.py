@@ -18,6 +18,8 @@ def _scene(which, w, h):
     if which == "mesh":
         return scenes.large_mesh(w, h, terrain_quads=48, instance_count=12, instance_frequency=8, glass_spheres=4,
                                  env_size=(64, 32))
+    if which == "spheres":  # no lights and no environment: shading without shadow rays
+        return scenes.sphere_field(w, h, frequency=8, seed=5)
     if which == "room":  # alpha-masked textures
         return scenes.textured_room(w, h)
     scene, cam = scenes.cornell_box(w, h)
@@ -27,7 +29,7 @@ def _scene(which, w, h):
     return scene, cam
 
 
-@pytest.mark.parametrize("which", ["cornell", "mesh", "room", "lists"])
+@pytest.mark.parametrize("which", ["cornell", "mesh", "spheres", "room", "lists"])
 @pytest.mark.parametrize("size", [(1, 1), (3, 5), (65, 33), (257, 129)])
 def test_frame_does_not_depend_on_launch_size(cuda, which, size):
     w, h = size

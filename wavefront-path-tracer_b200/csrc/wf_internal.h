@@ -104,6 +104,8 @@ struct wf_scene {
     }
     // ... and no material is alpha-textured: the Opaque<> kernels
     bool opaque() const { return !alpha_textures && listless(); }
+    // nothing that shading samples with a shadow ray: no lights and no environment
+    bool eventless() const { return view.light_count == 0 && view.punctual_count == 0 && !view.env.present; }
     bool textured = false;        // some material has a texture binding
     uint32_t material_categories = 0;  // bit k: some material has shading category k (material_category)
     wf::Box bounds{};

@@ -604,6 +604,7 @@ constexpr int kUnconditional = -1;
 template <typename Tally = NoTally>
 struct InlineSink {
     static constexpr bool kDeferredGather = false;  // caustic gathers run inline
+    static constexpr bool kEvents = true;           // the scene may hold lights or an environment
     const DeviceScene* scene;
     V3 radiance;
     bool killed;
@@ -626,8 +627,22 @@ struct InlineSink {
     }
 };
 
+// Scenes without lights, punctual lights, environment or photon map: shading
+// asks for no shadow ray, and every term counts at once.
+struct DirectSink {
+    static constexpr bool kDeferredGather = false;
+    static constexpr bool kEvents = false;
+    V3 radiance;
+    WF_DEV int request(V3, V3, float) { return kUnconditional; }
+    WF_DEV bool may_be_visible(int) const { return true; }
+    WF_DEV void term(V3 c, int) { radiance += c; }
+    WF_DEV void kill_if_visible(int) {}
+    WF_DEV void apply_kill(Path&) const {}
+};
+
 struct DeferredSink {
     static constexpr bool kDeferredGather = true;  // caustic gathers go to GatherQueue
+    static constexpr bool kEvents = true;
     GatherQueue gathers;
     // shadow queue
     float4* shadow_origin;   // origin xyz, t_max
@@ -833,7 +848,7 @@ WF_DEV void sample_direct_environment(const DeviceScene& s, const RenderParams& 
 // addEnvironmentOrSky, device_traversal.cuh:577-587.
 template <typename Sink>
 WF_DEV void add_environment_or_sky(const DeviceScene& s, const RenderParams& rp, const Path& path, Sink& sink) {
-    if (s.env.present) {
+    if (Sink::kEvents && s.env.present) {
         EnvUv at = environment_uv(s.env, path.direction);
         float weight =
             path.depth > 0 && !path.specular ? power_heuristic(path.prev_pdf, environment_pdf(s.env, at)) : 1.0f;
@@ -1124,7 +1139,7 @@ WF_DEV V3 continue_dielectric(const DeviceScene& s, const RenderParams& rp, Path
     DielectricInterface b = dielectric_interface(normalize(path.direction), hit.geometric_normal, shaded.normal, m.ior);
     float eta_sq = b.eta * b.eta;
     int reflection_test = kUnconditional, transmission_test = kUnconditional;
-    if (s.env.present && path.depth + 1 < rp.max_depth) {
+    if (Sink::kEvents && s.env.present && path.depth + 1 < rp.max_depth) {
         if (b.reflectance > 0.0f) {
             V3 d = b.reflection;
             reflection_test = sink.request(offset_ray_origin(hit.position, hit.geometric_normal, d, hit.t), d, 1.0e30f);
@@ -1217,7 +1232,7 @@ WF_DEV V3 continue_gltf(const DeviceScene& s, const RenderParams& rp, Path& path
     bool delta = (coat && g.coat_roughness <= 0) || (specular && g.roughness <= 0);
     int base_test = kUnconditional, coat_test = kUnconditional;
     V3 base_coefficient = pbr_base_fresnel(g, dot(pbr_specular_normal(g), view)) * (1.f - w.coat);
-    if (s.env.present && path.depth + 1 < rp.max_depth) {
+    if (Sink::kEvents && s.env.present && path.depth + 1 < rp.max_depth) {
         for (int lobe = 0; lobe < 2; ++lobe) {
             bool is_coat = lobe == 1;
             float mass = is_coat ? w.coat : w.specular;
@@ -1359,7 +1374,8 @@ WF_DEV bool shade_path(const DeviceScene& s, const RenderParams& rp, Path& path,
     // and the environment before its continuation (the same order in each
     // material branch of shadePaths); one call site keeps the kernel small.
     bool gltf = (m.flags & kMatGltfPbr) != 0;
-    if (gltf || type == kDiffuse || type == kSpecGloss || (type == kMetal && roughness > 0.0f)) {
+    if (Sink::kEvents &&
+        (gltf || type == kDiffuse || type == kSpecGloss || (type == kMetal && roughness > 0.0f))) {
         sample_direct_light(s, rp, path, hit, shaded, m, sink);
         sample_direct_punctual(s, rp, path, hit, shaded, m, sink);
         sample_direct_environment(s, rp, path, hit, shaded, m, sink);
@@ -1367,7 +1383,7 @@ WF_DEV bool shade_path(const DeviceScene& s, const RenderParams& rp, Path& path,
     if (gltf) {
         direction = continue_gltf(s, rp, path, hit, shaded, m, sink);
     } else if (type == kDiffuse) {
-        if (rp.photons.enabled) {
+        if (Sink::kEvents && rp.photons.enabled) {
             if constexpr (Sink::kDeferredGather) {
                 sink.gather(path, shaded, albedo);
             } else {
