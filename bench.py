@@ -144,9 +144,11 @@ class ClockSampler:
 
 def algorithmic_bytes(profile, kernel):
     """Algorithmic bytes of one kernel's launches in the profiled pass.
-    Per ray state: 32 B ray in + 16 B hit/result out.  Traversal: 32 B per
-    node visit (one pair of child boxes), 48 B per triangle test, 16 B per
+    Per ray state: 32 B ray in + 16 B hit/result out.  Traversal: 80 B per
+    node visit of the 8-wide BVH (shadow rays), 64 B where camera rays' visits
+    of two-box nodes are counted in (trace), 48 B per triangle test, 16 B per
     sphere test, 64 B per instance entry."""
+    node_bytes = 64 if kernel == "trace" else 80
     if kernel == "trace":
         rays, nodes, tris, sph, inst = (profile["extension_rays"], profile["closest_nodes"],
                                         profile["closest_triangles"], profile["closest_spheres"],
@@ -154,7 +156,7 @@ def algorithmic_bytes(profile, kernel):
     else:
         rays, nodes, tris, sph, inst = (profile["shadow_rays"], profile["any_nodes"], profile["any_triangles"],
                                         profile["any_spheres"], profile["any_instances"])
-    return 48 * rays + 32 * nodes + 48 * tris + 16 * sph + 64 * inst
+    return 48 * rays + node_bytes * nodes + 48 * tris + 16 * sph + 64 * inst
 
 
 def ncu_summary(kernel, workload):

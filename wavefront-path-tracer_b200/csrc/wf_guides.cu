@@ -54,9 +54,11 @@ WF_DEV bool closest_surface(const DeviceScene& s, V3 o, V3 d, SurfaceHit& sh) {
     return finish_hit(s, o, d, h.t, h.u, h.v, h.prim, h.inst, sh);
 }
 
-// Bounded to 8 CTAs of 128 per SM (64 registers, 64 B of spill): a 1080p
-// guide frame of the large mesh takes 3.51 ms, against 4.12 ms unbounded (80
-// registers, 6 CTAs) and 3.78 ms at 72 registers.
+// Bounded to 8 CTAs of 128 per SM (64 registers, 60 B of spill): a 1080p
+// guide frame of the large mesh took 3.51 ms, against 4.12 ms unbounded (80
+// registers, 6 CTAs) and 3.78 ms at 72 registers, all with a warp's pixels in
+// a row; in blocks of 8 x 4 the bounded kernel went from 2.92 to 2.32 ms at
+// the frame it is timed on (700 k triangles, download included).
 __global__ void __launch_bounds__(128, 8) k_frame_guides(const __grid_constant__ DeviceScene s, Camera camera,
                                                       Camera previous, uint32_t has_previous, uint32_t width,
                                                       uint32_t height, uint32_t x0, uint32_t y0, uint32_t tile_w,

@@ -202,10 +202,10 @@ WF_DEV void trace_stage(const DeviceScene& s, PathSoA ps, const uint32_t* queue,
     if constexpr (Tally::kCounts) flush_tally(tally, totals);
 }
 
-// Lane-refill bounces: at most 72 registers (7 CTAs of 128 per SM): 8 bytes
-// of spill cost less than the warps a 79-register allocation (6 CTAs) leaves
-// out; a 64-register cap spills far more.  __maxnreg__ keeps every block
-// size launchable.
+// Lane-refill bounces: at most 64 registers (8 CTAs of 128 per SM).  Bound by
+// the latency of a lane's chain of node fetches; 56, 64 and 72 registers
+// measured alike (1080p large mesh, 4 samples: 68.5 ms within 0.5 %).
+// __maxnreg__ keeps every block size launchable.
 template <typename Tally, bool kLanes = true>
 __global__ void __maxnreg__(64) k_trace(const __grid_constant__ DeviceScene s, PathSoA ps, const uint32_t* queue, const uint32_t* count,
                                         float4* hit_a, uint32_t* hit_inst, Counters* c, uint32_t bounce,

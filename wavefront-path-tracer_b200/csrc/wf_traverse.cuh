@@ -1,4 +1,5 @@
-// Closest-hit and any-hit traversal.
+// Closest-hit and any-hit traversal of the BVH2s: camera rays, frame guides
+// and the rays that the 8-wide BVH's traversal leaves undecided (wf_wide.cuh).
 //
 // Semantics follow the reference's traceRay / isOccluded
 // (include/renderer/device_traversal.cuh:1035-1184) exactly: the same visit

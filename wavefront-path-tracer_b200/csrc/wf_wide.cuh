@@ -1,6 +1,7 @@
 // Traversal of the compressed 8-wide BVHs (WideNode, wf_device.cuh): closest
 // hit and any hit as resumable per-lane state machines, used by every kernel
-// that traces rays.
+// that traces rays but camera rays and frame guides, whose warps visit the
+// same BVH2 nodes together.
 //
 // The node layout and the test of eight quantised child boxes against a
 // ray-order hit mask follow Ylitie, Karras and Laine, "Efficient Incoherent
