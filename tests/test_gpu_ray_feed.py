@@ -84,3 +84,28 @@ def test_large_ray_batches_match_small_ones(cuda, which):
         assert dev.trace_closest(rays[:count]).tobytes() == hits[:count].tobytes()
         assert np.array_equal(dev.trace_any(rays[:count], limit[:count]), occluded[:count])
     dev.close()
+
+
+@pytest.mark.parametrize("capacity,pass_paths", [(0, 0), (33, 0), (300, 1021)])
+def test_batch_of_scenes_without_lights(cuda, capacity, pass_paths):
+    """A batch of sphere fields shades without shadow rays; its images are
+    those of the streaming schedule, which always queues them."""
+    jobs, want = [], []
+    for w, h, depth, count, seed in ((31, 17, 6, 3, 1), (64, 40, 16, 2, 2), (1, 1, 1, 5, 3)):
+        scene, cam = scenes.sphere_field(w, h, frequency=8, seed=seed)
+        dev = wfpt.DeviceScene(scene)
+        jobs.append(dict(scene=dev, camera=cam, sample_start=7, sample_count=count,
+                         config=wfpt.render_config(w, h, max_depth=depth)))
+        r = wfpt.Renderer(dev, cam, wfpt.render_config(w, h, max_depth=depth, mode=abi.MODE_STREAM))
+        want.append(r.render_task((0, 0, w, h), 7, count))
+        r.close()
+    batch = wfpt.Batch(jobs, slot_capacity=capacity, pass_paths=pass_paths)
+    for _ in range(2):
+        batch.reset()
+        batch.run()
+        batch.synchronize()
+        for k, image in enumerate(want):
+            assert np.array_equal(batch.download(k).view(np.uint32), image.view(np.uint32))
+    batch.close()
+    for job in jobs:
+        job["scene"].close()

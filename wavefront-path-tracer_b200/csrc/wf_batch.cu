@@ -57,6 +57,7 @@ struct wf_batch {
     bool own_stream = false;
     bool opaque = true;     // every job's scene is (wf_scene::opaque): the Opaque<> trace and shadow kernels
     bool textured = false;  // some job's scene has textured materials: k_batch_shade<true>
+    bool direct = true;     // every job's scene is eventless (wf_scene::eventless): k_batch_shade_direct
     int device = 0, sm_count = 148;
     std::vector<void*> allocations;
     std::vector<wf_batch_job> jobs;
@@ -164,7 +165,7 @@ __global__ void k_batch_accumulate(BatchView b, const Counters* c) {
     }
 }
 
-// At most 72 registers, as k_trace (7 CTAs of 128 per SM instead of 6).
+// At most 64 registers (8 CTAs of 128 per SM), as k_trace.
 template <typename Tally>
 __global__ void __maxnreg__(64) k_batch_trace(BatchView b, PathSoA ps, const uint32_t* queue, const uint32_t* count, float4* hit_a,
                               uint32_t* hit_inst, Counters* c, uint32_t refill_at) {
@@ -176,6 +177,7 @@ __global__ void __maxnreg__(64) k_batch_trace(BatchView b, PathSoA ps, const uin
         c->gather_count = 0;
         c->work_shade = 0;
         c->extension_rays += n;
+        c->queue_count[count == &c->queue_count[0] ? 1 : 0] = 0;  // the next queue (k_batch_shade_direct fills it)
     }
     Tally tally;
     Lane L;
@@ -314,6 +316,74 @@ __global__ void __maxnreg__(64) k_batch_shadow(BatchView b, const float4* shadow
     }
 }
 
+// The end of a bounce for a warp's slots: slots whose path has ended start the
+// pass's next units, and the slots that carry a path enter the next queue.
+WF_DEV void batch_continue(const BatchView& b, const PathSoA& ps, uint32_t p, bool alive, bool need_unit,
+                           uint32_t* next, uint32_t* next_count, uint32_t capacity, Counters* c) {
+    uint32_t lane = threadIdx.x & 31;
+    unsigned want = __ballot_sync(0xffffffffu, need_unit);
+    if (want) {
+        uint32_t first = 0;
+        if (lane == 0) first = atomicAdd(&c->next_unit, uint32_t(__popc(want)));
+        first = __shfl_sync(0xffffffffu, first, 0);
+        if (need_unit) {
+            uint32_t unit = first + __popc(want & ((1u << lane) - 1u));
+            if (unit < c->pass_end) {
+                batch_start(b, ps, p, unit);
+                alive = true;
+            }
+        }
+    }
+    unsigned mask = __ballot_sync(0xffffffffu, alive);
+    uint32_t out = 0;
+    if (lane == 0 && mask) out = atomicAdd(next_count, uint32_t(__popc(mask)));
+    out = __shfl_sync(0xffffffffu, out, 0);
+    uint32_t rank = __popc(mask & ((1u << lane) - 1u));
+    if (alive && out + rank < capacity) next[out + rank] = p;
+}
+
+// Shading when no job's scene has anything that a shadow ray is asked for
+// (wf_scene::eventless), as k_shade_direct: terms count at once, and the
+// bounce ends here without the shadow and finalize kernels.  Eight uneven
+// sphere field jobs: 4.28 -> 3.71 ms.
+template <bool kTextures>
+__global__ void __launch_bounds__(128, 4) k_batch_shade_direct(BatchView b, PathSoA ps, const uint32_t* queue,
+                                                               const uint32_t* count, const float4* hit_a,
+                                                               const uint32_t* hit_inst, Counters* c, uint32_t* next,
+                                                               uint32_t* next_count, uint32_t capacity) {
+    count_launch(c);
+    uint32_t n = *count;
+    uint32_t lane = threadIdx.x & 31;
+    if (blockIdx.x == 0 && threadIdx.x == 0) c->work_trace = 0;
+    uint32_t base;
+    while (next_chunk(&c->work_shade, n, base)) {
+        uint32_t i = base + lane;
+        bool alive = false, need_unit = false;
+        uint32_t p = 0;
+        if (i < n) {
+            p = queue[i];
+            const BatchJob& J = b.jobs[b.slot_job[p]];
+            Path path = load_path(ps, p);
+            float4 ha = hit_a[i];
+            SurfaceHit sh;
+            bool did_hit = finish_hit(J.scene, path.origin, path.direction, ha.x, ha.y, ha.z, __float_as_uint(ha.w),
+                                      hit_inst[i], sh);
+            DirectSink sink;
+            sink.radiance = f4xyz(ps.radiance[p]);
+            alive = shade_path<DirectSink, kTextures>(J.scene, J.rp, path, did_hit, sh, sink);
+            V3 rad = sink.radiance;
+            if (alive) {
+                store_path(ps, p, path);
+                ps.radiance[p] = make_float4(rad.x, rad.y, rad.z, 0.0f);
+            } else {
+                b.unit_radiance[b.slot_unit[p] - c->pass_begin] = make_float4(rad.x, rad.y, rad.z, 0.0f);
+                need_unit = true;
+            }
+        }
+        batch_continue(b, ps, p, alive, need_unit, next, next_count, capacity, c);
+    }
+}
+
 // Term accumulation, kill rule and compaction as in the single-scene
 // finalize; an ended path stores its radiance by unit (k_batch_accumulate
 // adds it after the pass), then its slot starts the pass's next unit.
@@ -348,25 +418,7 @@ __global__ void k_batch_finalize(BatchView b, PathSoA ps, const uint32_t* queue,
                 need_unit = true;
             }
         }
-        unsigned want = __ballot_sync(0xffffffffu, need_unit);
-        if (want) {
-            uint32_t first = 0;
-            if (lane == 0) first = atomicAdd(&c->next_unit, uint32_t(__popc(want)));
-            first = __shfl_sync(0xffffffffu, first, 0);
-            if (need_unit) {
-                uint32_t unit = first + __popc(want & ((1u << lane) - 1u));
-                if (unit < c->pass_end) {
-                    batch_start(b, ps, p, unit);
-                    alive = true;
-                }
-            }
-        }
-        unsigned mask = __ballot_sync(0xffffffffu, alive);
-        uint32_t out = 0;
-        if (lane == 0 && mask) out = atomicAdd(next_count, uint32_t(__popc(mask)));
-        out = __shfl_sync(0xffffffffu, out, 0);
-        uint32_t rank = __popc(mask & ((1u << lane) - 1u));
-        if (alive && out + rank < capacity) next[out + rank] = p;
+        batch_continue(b, ps, p, alive, need_unit, next, next_count, capacity, c);
     }
 }
 
@@ -463,6 +515,17 @@ wf_status capture_batch(wf_batch* b) {
         else
             k_batch_trace<NoTally><<<batch_grid(b, 0, cap, b->block), b->block, 0, st>>>(
                 b->view, b->paths, b->queue[cur], cur_count, b->hit_a, b->hit_inst, b->counters, b->refill);
+        if (b->direct) {
+            if (b->textured)
+                k_batch_shade_direct<true><<<batch_grid(b, 1, cap, 128), 128, 0, st>>>(
+                    b->view, b->paths, b->queue[cur], cur_count, b->hit_a, b->hit_inst, b->counters, b->queue[nxt],
+                    next_count, cap);
+            else
+                k_batch_shade_direct<false><<<batch_grid(b, 1, cap, 128), 128, 0, st>>>(
+                    b->view, b->paths, b->queue[cur], cur_count, b->hit_a, b->hit_inst, b->counters, b->queue[nxt],
+                    next_count, cap);
+            continue;
+        }
         if (b->textured)
             k_batch_shade<true><<<batch_grid(b, 1, cap, 128), 128, 0, st>>>(
                 b->view, b->paths, b->queue[cur], cur_count, b->hit_a, b->hit_inst, b->terms, b->shade_out,
@@ -555,6 +618,7 @@ wf_status batch_create(const wf_batch_job* jobs, uint32_t count, const wf_batch_
     for (uint32_t i = 0; i < count; ++i) {
         b->opaque = b->opaque && jobs[i].scene->opaque();
         b->textured = b->textured || jobs[i].scene->textured;
+        b->direct = b->direct && jobs[i].scene->eventless();
     }
 
     // Unit order: job by job, in the given order or longest per-pixel work first.
@@ -653,8 +717,12 @@ wf_status batch_create(const wf_batch_job* jobs, uint32_t count, const wf_batch_
     b->view.pixels = uint32_t(pixels_total);
     WF_BATCH_CUDA(b->opaque ? batch_resident(bp, 0, k_batch_trace<Opaque<NoTally>>, b->block)
                             : batch_resident(bp, 0, k_batch_trace<NoTally>, b->block));
-    WF_BATCH_CUDA(b->textured ? batch_resident(bp, 1, k_batch_shade<true>, 128)
-                              : batch_resident(bp, 1, k_batch_shade<false>, 128));
+    if (b->direct)
+        WF_BATCH_CUDA(b->textured ? batch_resident(bp, 1, k_batch_shade_direct<true>, 128)
+                                  : batch_resident(bp, 1, k_batch_shade_direct<false>, 128));
+    else
+        WF_BATCH_CUDA(b->textured ? batch_resident(bp, 1, k_batch_shade<true>, 128)
+                                  : batch_resident(bp, 1, k_batch_shade<false>, 128));
     WF_BATCH_CUDA(b->opaque ? batch_resident(bp, 2, k_batch_shadow<Opaque<NoTally>>, b->block)
                             : batch_resident(bp, 2, k_batch_shadow<NoTally>, b->block));
     WF_BATCH_CUDA(batch_resident(bp, 3, k_batch_finalize, 256));
