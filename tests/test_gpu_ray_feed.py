@@ -22,6 +22,17 @@ def _scene(which, w, h):
         return scenes.sphere_field(w, h, frequency=8, seed=5)
     if which == "room":  # alpha-masked textures
         return scenes.textured_room(w, h)
+    if which == "contact":  # glass cubes on an instanced floor, seen from among them: faces on one plane
+        scene = wfpt.Scene()
+        rng = np.random.default_rng(5)
+        mats = [scene.add_material(wfpt.material(t, c, ior=1.5)) for t, c in
+                ((abi.MAT_DIFFUSE, (0.6, 0.5, 0.4)), (abi.MAT_DIELECTRIC, (1, 1, 1)), (abi.MAT_DIFFUSE, (0.2, 0.6, 0.3)))]
+        scene.add_mesh(scenes.box((0, 0, 0), (1, 1, 1), 0, mats[0]))
+        scene.instances = np.concatenate(
+            [scenes.instance(0, (0, -10, 0), 20.0)] +
+            [scenes.instance(0, (x, 0.5, z), 1.0, 0.0, mats[1 + k % 2])
+             for k, (x, z) in enumerate(rng.uniform(-6, 6, (60, 2)))])
+        return scene, scenes.look_at_camera((0.494, 0.02, 6.4), (0.45, -0.3, 6.2), 90.0, w, h)
     scene, cam = scenes.cornell_box(w, h)
     if which == "lists":  # primitives outside the BVHs: the generic kernels
         scene.static_triangles = scenes.quad((-1, 0, 1), (1, 0, 1), (1, 0.5, 1), (-1, 0.5, 1), 1)
@@ -29,7 +40,7 @@ def _scene(which, w, h):
     return scene, cam
 
 
-@pytest.mark.parametrize("which", ["cornell", "mesh", "spheres", "room", "lists"])
+@pytest.mark.parametrize("which", ["cornell", "mesh", "spheres", "room", "lists", "contact"])
 @pytest.mark.parametrize("size", [(1, 1), (3, 5), (65, 33), (257, 129)])
 def test_frame_does_not_depend_on_launch_size(cuda, which, size):
     w, h = size

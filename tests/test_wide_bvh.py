@@ -7,7 +7,8 @@ agree bit for bit.  The rays are those where the two could part: axis-parallel
 ones with zero and denormal components, origins on box planes, through shared
 vertices and edges, grazing, from far away and from inside, with directions of
 other lengths than 1; the scenes flat, degenerate, duplicated, tiny, huge,
-scaled instances, and past the range the wide test covers."""
+scaled instances, instances and spheres that touch one another, and past the
+range the wide test covers."""
 import ctypes as C
 import shutil
 import subprocess
@@ -182,6 +183,118 @@ def test_instances_spheres_and_direct_lists(check):
     only.add_material(material(abi.MAT_DIFFUSE, (0.5, 0.5, 0.5)))
     only.triangles = scenes.triangles(v[:, 0], v[:, 1], v[:, 2], 0)  # the direct list's own BVH
     check(only, hard_rays(v.reshape(-1, 3), 1.0, 16, 8000))
+
+
+def unit(d):
+    return (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+
+
+def touching_scene(offset, floor_yaw=0.0, box_yaw=0.0, stack=0, scale=20.0, seed=0):
+    """Unit cubes that stand on a scaled cube (its top is y = 0 before the
+    offset) and on one another, every one an instance of one mesh."""
+    rng = np.random.default_rng(seed)
+    s = Scene()
+    s.add_material(material(abi.MAT_DIFFUSE, (0.5, 0.5, 0.5)))
+    s.add_mesh(scenes.box((0, 0, 0), (1, 1, 1), 0, 0))
+    inst = [scenes.instance(0, np.add(offset, (0, -scale / 2, 0)), scale, floor_yaw)]
+    for _ in range(40):
+        x, z = rng.uniform(-0.4 * scale, 0.4 * scale, 2)
+        inst.append(scenes.instance(0, np.add(offset, (x, 0.5, z)), 1.0, box_yaw * rng.random()))
+        for k in range(stack):
+            x, z = x + 0.2 * rng.normal(), z + 0.2 * rng.normal()
+            inst.append(scenes.instance(0, np.add(offset, (x, 1.5 + k, z)), 1.0, box_yaw * rng.random()))
+    s.instances = np.concatenate(inst)
+    return s
+
+
+@pytest.mark.parametrize("offset", [(0, 0, 0), (100, 3, -50), (1e4, 1e3, -3e3)])
+@pytest.mark.parametrize("floor_yaw,box_yaw,stack", [(0.0, 0.0, 0), (0.0, 90.0, 2), (30.0, 90.0, 0)])
+def test_touching_instances(check, offset, floor_yaw, box_yaw, stack):
+    """Faces that share a plane with other instances' boxes: there the TLAS
+    leaf's entry (world ray) and the hit's distance (local ray) round apart,
+    and the BVH2's culling order decides.  Rays start within 5 cm of the
+    contact plane, as bounces near a contact do, some of them grazing it."""
+    s = touching_scene(offset, floor_yaw, box_yaw, stack)
+    rng = np.random.default_rng(7)
+    n = 100_000
+    o = rng.uniform(-9, 9, (n, 3))
+    o[:, 1] = rng.uniform(0, 0.05, n) + rng.integers(0, stack + 1, n)
+    d = rng.normal(0, 1, (n, 3))
+    d[::3, 1] *= 10.0 ** rng.uniform(-3, 0, len(d[::3]))
+    got = check(s, make_rays(o + offset, unit(d)))
+    assert got["usable"] == 1 and got["hits"] > n // 3
+
+
+def test_touching_primitives_of_several_kinds(check):
+    """An instance's faces on a static quad's plane, a direct list's and a
+    sphere's, and a sphere on the floor instance."""
+    for kind in ("static", "list", "sphere", "direct sphere"):
+        s = touching_scene((0, 0, 0), box_yaw=45.0)
+        floor = scenes.quad((-9, 0, 9), (9, 0, 9), (9, 0, -9), (-9, 0, -9), 0)
+        if kind == "static":
+            s.static_triangles = floor
+        elif kind == "list":
+            s.triangles = floor
+        else:
+            sp = np.zeros(60, abi.SPHERE_DTYPE)
+            sp["center"] = np.random.default_rng(1).uniform(-8, 8, (60, 3))
+            sp["radius"] = 0.4
+            sp["center"][:, 1] = 0.4
+            sp["accel"] = abi.ACCEL_BVH if kind == "sphere" else abi.ACCEL_DIRECT
+            s.spheres = sp
+        rng = np.random.default_rng(8)
+        o = rng.uniform(-9, 9, (60_000, 3))
+        o[:, 1] = rng.uniform(0, 0.05, len(o))
+        check(s, make_rays(o, unit(rng.normal(0, 1, o.shape))))
+
+
+@pytest.mark.parametrize("radius,ground,near,far", [(0.2, 1000.0, 1e-2, 20.0), (0.2, 1000.0, 20.0, 2e3),
+                                                    (0.02, 0.0, 1.0, 1e3), (0.2, 0.0, 1e2, 1e4),
+                                                    (5.0, 0.0, 1e-2, 100.0)])
+def test_spheres_from_near_and_far(check, radius, ground, near, far):
+    """Small spheres that touch, on a large one: from many radii away the
+    discriminant cancels and a hit can lie before the sphere's box."""
+    rng = np.random.default_rng(3)
+    n = 400
+    c = rng.uniform(-11, 11, (n, 3))
+    c[:, 1] = radius
+    turn = rng.uniform(0, 6.3, n // 2)
+    c[n // 2:] = c[:n // 2] + 2 * radius * np.stack([np.cos(turn), 0 * turn, np.sin(turn)], 1)
+    s = Scene()
+    s.add_material(material(abi.MAT_DIFFUSE, (0.5, 0.5, 0.5)))
+    sp = np.zeros(n + (ground > 0), abi.SPHERE_DTYPE)
+    sp["center"][:n], sp["radius"][:n] = c, radius
+    if ground:
+        sp[n] = ((0, -ground, 0), ground, 0, abi.ACCEL_BVH)
+    sp["accel"] = abi.ACCEL_BVH
+    s.spheres = sp
+    k = 150_000
+    at = c[rng.integers(0, n, k)] + radius * unit(rng.normal(0, 1, (k, 3)))
+    d = rng.normal(0, 1, (k, 3))
+    d[:, 1] = -np.abs(d[:, 1]) * 10.0 ** rng.uniform(-2, 0, k)
+    d = unit(d)
+    t = np.exp(rng.uniform(np.log(near), np.log(far), (k, 1)))
+    check(s, make_rays((at + 0.02 * radius * rng.normal(0, 1, (k, 3)) - d * t).astype(np.float32), d))
+
+
+@pytest.mark.parametrize("kind,usable", [("sheared", 1), ("strongly sheared", 1), ("not inverse", 0)])
+def test_other_instance_transforms(check, kind, usable):
+    """Scales after a rotation (|L| |W| of 3, 60 and more than the margins can
+    hold), and a world-to-local matrix that is not the other's inverse."""
+    s = touching_scene((0, 0, 0), box_yaw=90.0)
+    inst = s.instances.copy()
+    l2w = inst["local_to_world"].astype(np.float64)
+    stretch = {"sheared": 1.5, "strongly sheared": 30.0, "not inverse": 1.0}[kind]
+    l2w[1:, :, 0] *= stretch                                # rows of images: scales world x
+    inst["local_to_world"] = l2w.astype(np.float32)
+    inst["world_to_local"] = np.linalg.inv(l2w).astype(np.float32)
+    if kind == "not inverse":
+        inst["world_to_local"][3] *= np.float32(1.01)
+    s.instances = inst
+    rng = np.random.default_rng(9)
+    o = rng.uniform(-9, 9, (60_000, 3))
+    o[:, 1] = rng.uniform(0, 0.05, len(o))
+    assert check(s, make_rays(o, unit(rng.normal(0, 1, o.shape))))["usable"] == usable
 
 
 def test_repository_scenes(check):

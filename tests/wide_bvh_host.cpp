@@ -40,7 +40,7 @@ void build_wide(Built& b) {
         uint32_t item = trees[i].root < 0 ? (kLeafItem | uint32_t(~trees[i].root)) : uint32_t(trees[i].root);
         items.push_back(item | (i == b.h.tlas.wide ? kTlasItem : 0u));
     }
-    bool usable = true;
+    bool usable = b.h.margins.usable != 0;
     std::vector<uint2> bases;
     uint32_t triangle_count = 0, leaf_count = 0;
     for (uint32_t i = 0; i < items.size(); ++i) {
@@ -83,6 +83,7 @@ void build_wide(Built& b) {
     v.direct_sphere_count = uint32_t(b.h.direct_spheres.size());
     v.direct_instance_count = uint32_t(b.h.direct_instances.size());
     v.any_alpha_reject = b.h.any_alpha_reject ? 1u : 0u;
+    v.wide = b.h.margins;
     b.triangles.resize(triangle_count);
     b.leaves.resize(leaf_count);
     for (uint32_t i = 0; i < items.size(); ++i) {
@@ -91,7 +92,10 @@ void build_wide(Built& b) {
         b.nodes.push_back(wide_record(v, c, (items[i] & kTlasItem) != 0, bases[i].x, bases[i].y, b.triangles.data(),
                                       b.leaves.data()));
     }
-    v.wide = WideBvh{b.nodes.data(), b.triangles.data(), b.leaves.data(), usable && !trees.empty() ? 1u : 0u};
+    v.wide.nodes = b.nodes.data();
+    v.wide.triangles = b.triangles.data();
+    v.wide.leaves = b.leaves.data();
+    v.wide.usable = usable && !trees.empty() ? 1u : 0u;
 }
 }  // namespace
 

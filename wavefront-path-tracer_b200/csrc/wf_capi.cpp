@@ -176,6 +176,7 @@ wf_status wf_scene_create(const wf_scene_desc* desc, wf_scene** out) {
     number(h.direct_bvh);
     number(h.tlas);
     uint32_t tlas_tree = h.tlas.wide;
+    v.wide = h.margins;
     up(&v.triangles, h.triangles);
     up(&v.normals, h.normals);
     up(&v.nodes, h.nodes);

@@ -152,11 +152,20 @@ static_assert(sizeof(WideLeaf) == 112, "TLAS leaf record");
 // (wf_wide.cuh); larger scenes use the BVH2s alone.
 constexpr float kWideMaxCoordinate = 1.0e7f;
 
+// Least values of WideBvh's margins, and the largest reach with which culling
+// is still worth its nodes (a matrix and its inverse 1/2048 apart).
+constexpr float kWideReach = 1.0f / 32768.0f, kWideSphereReach = 1.0f / 8192.0f, kWideMaxReach = 1.0f / 512.0f;
+constexpr float kWideSlack = 1.0f + 1.0f / 32768.0f, kWideSphereSlack = 1.0f + 1.0f / 64.0f;
+
 struct WideBvh {
     const WideNode* nodes;
     const WideTriangle* triangles;
     const WideLeaf* leaves;
     uint32_t usable;  // 0: some box is not finite or beyond kWideMaxCoordinate
+    // how far before its box a closest hit of the TLAS may lie (wf_wide.cuh):
+    // a part of the distance to the farthest corner, a world distance, and a
+    // factor on the closest distance so far
+    float reach, base, slack;
 };
 
 // Triangle .w lanes: a.w = original index | kTriHasNormals, b.w = material,

@@ -44,6 +44,7 @@ struct HostScene {
     std::vector<Punctual> punctual;
     uint32_t directional_count = 0;
     BvhRef tlas{kNoRoot, {}, kNoWide};
+    WideBvh margins;  // the wide traversal's reach, base and slack; usable 0: past what they can hold
     BvhRef direct_bvh{kNoRoot, {}, kNoWide};
     uint32_t static_first = 0, static_count = 0;
     uint32_t direct_first = 0, direct_count = 0;

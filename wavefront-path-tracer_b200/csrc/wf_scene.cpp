@@ -236,6 +236,34 @@ wf_status fail(wf_status status, const char* format, ...) {
 
 const char* last_error_text() { return g_error.c_str(); }
 
+// How far the world box of an instance and the distances found in its own
+// frame may part (wf_wide.cuh): the rounding of the ray's transform grows with
+// |L| |W| (local to world times world to local), and a W that is not quite L's
+// inverse moves the ray by L W - I.
+static void instance_margins(const wf_instance& in, const BvhBox& box, WideBvh& m) {
+    double condition = 0.0, residual = 0.0, far = 0.0;
+    for (int row = 0; row < 3; ++row) {
+        double sum = 0.0, off = 0.0;
+        for (int col = 0; col < 3; ++col) {
+            double v = row == col ? -1.0 : 0.0;
+            for (int k = 0; k < 3; ++k) {
+                double p = double(in.local_to_world[k][row]) * double(in.world_to_local[col][k]);
+                sum += std::fabs(p);
+                v += p;
+            }
+            off += std::fabs(v);
+        }
+        condition = std::max(condition, sum);
+        residual = std::max(residual, off);
+        far = std::max(far, std::fabs(double(in.translation[row])) +
+                                std::max(std::fabs(double(box.lo[row])), std::fabs(double(box.hi[row]))));
+    }
+    double reach = std::max(double(kWideReach) * std::max(1.0, condition / 8.0), 4.0 * residual);
+    if (!(reach <= kWideMaxReach) || !(far <= 4.0 * kWideMaxCoordinate)) m.usable = 0;
+    m.reach = fmaxf(m.reach, float(reach));
+    m.base = fmaxf(m.base, float(0.25 * reach * far));
+}
+
 wf_status build_host_scene(const wf_scene_desc* d, HostScene& s) {
     if (!d) return fail(WF_ERR_INVALID_ARG, "scene description is null");
     auto need = [](const void* p, uint32_t n) { return n == 0 || p != nullptr; };
@@ -444,6 +472,7 @@ wf_status build_host_scene(const wf_scene_desc* d, HostScene& s) {
     }
 
     // --- spheres + TLAS (uploadSceneTlas, scene.cu:175-239)
+    s.margins = WideBvh{nullptr, nullptr, nullptr, 1u, kWideReach, 0.0f, kWideSlack};
     std::vector<BvhBox> leaf_boxes;
     for (uint32_t i = 0; i < d->sphere_count; ++i) {
         const wf_sphere& sp = d->spheres[i];
@@ -463,6 +492,8 @@ wf_status build_host_scene(const wf_scene_desc* d, HostScene& s) {
         grow(s.bounds, b);
         leaf_boxes.push_back(b);
         s.tlas_leaves.push_back(0x80000000u | i);
+        s.margins.reach = fmaxf(s.margins.reach, kWideSphereReach);
+        s.margins.slack = kWideSphereSlack;
     }
     for (uint32_t i = 0; i < d->instance_count; ++i) {
         const wf_instance& in = d->instances[i];
@@ -486,6 +517,7 @@ wf_status build_host_scene(const wf_scene_desc* d, HostScene& s) {
         grow(s.bounds, w);
         leaf_boxes.push_back(w);
         s.tlas_leaves.push_back(i);
+        instance_margins(in, w, s.margins);
     }
     if (!leaf_boxes.empty()) {
         build_bvh(leaf_boxes.data(), uint32_t(leaf_boxes.size()), bin);

@@ -10,23 +10,47 @@
 // lanes; an 8-wide node takes the place of about three BVH2 levels, so a ray
 // makes a third of the fetches and loop turns.
 //
-// Same results, bit for bit, as the reference's BVH2 traversal (traceRay /
-// isOccluded, device_traversal.cuh:1035-1184; trace_closest_binary and
-// trace_any_binary here).  The wide boxes contain the BVH2's boxes, so a
-// candidate the BVH2 meets is met here too; what is left is:
-//   * Candidates the BVH2 never tests because a box on the way misses.  The
-//     slab test's operations are monotone in the box planes, so a leaf is
-//     reached in the BVH2 exactly when its own box passes, which
-//     `exact_box` checks, in the BVH2's arithmetic, before a candidate
-//     counts.
-//   * The visit order.  The BVH2 keeps the first of two equal distances, and
-//     its "entry < closestT" culling can drop a candidate whose box entry
-//     rounds past its own distance.  Both need two candidates whose
-//     distances agree to within kNear (or a box entry further past its
-//     candidate than that): such rays are traced once more by
-//     trace_closest_binary.  Rays through a shared edge of two triangles are
-//     the usual case, about one in 10^5 or fewer.
-//   * Any-hit queries do not depend on the order.
+// Same results as the reference's BVH2 traversal (traceRay / isOccluded,
+// device_traversal.cuh:1035-1184; trace_closest_binary and trace_any_binary
+// here).  A candidate is a primitive whose own test and whose boxes' slab
+// tests pass, the closest distance left aside.  The slab test's operations
+// are monotone in the box planes, so the boxes of one BVH2 pass exactly when
+// the leaf's does: exact_leaf_box and exact_triangle_box check it, in the
+// BVH2's arithmetic, for the TLAS leaf and for the triangle.  The BVH2 also
+// culls by "entry < closestT", in its own visit order.  Its answer is the
+// closest candidate whatever the order when the entries of that candidate's
+// boxes (the TLAS leaf's, of the world ray, and the triangle's, of the local
+// one) lie before the distance of every other candidate.  So a ray whose
+// closest candidate has an entry, or another candidate, that is not clearly
+// (kNear) on its side is traced once more by trace_closest_binary.  Rays
+// through a shared edge of two triangles and rays between touching surfaces
+// are the usual cases.  Any-hit queries do not depend on the order.
+//
+// Nodes are culled here only where no candidate below them can be the
+// closest.  A candidate's computed distance may lie before its own box, by
+// the rounding of its test, so the entry that culls is that of a box grown by
+// the errors below (WideRay::margin); the boxes' own tests are not widened.
+//   * A triangle's distance is that of a triangle moved by a few roundings of
+//     the vector from the ray's origin to it (some 24 u / sin of its sharpest
+//     corner at most, u = 2^-24): 2^-15 of the distance to the farthest
+//     corner of the BVH's box, which leaves room for corners down to 3
+//     degrees.
+//     Not covered: a ray within about a degree of the triangle's plane that
+//     meets it within rounding of the edge of its box, in front of a surface
+//     closer than that error; such a ray may keep that surface's hit where
+//     the BVH2's order finds the triangle's.
+//   * An instance's distance is found in its own frame.  Its world box is off
+//     by the roundings of the ray's transform, 8 u |L| |W| (local to world,
+//     world to local) times the distance, and of the translation and the box
+//     itself: WideBvh::reach and ::base, from the scene's instances.
+//   * A sphere's discriminant cancels: its distance is that of a sphere whose
+//     squared radius is off by 12 u of its squared distance.  Up to 295 radii
+//     away that is less than 2^-13 of the distance on the radius (reach);
+//     beyond, box and sphere together are 2^-6 of the distance
+//     (WideBvh::slack).
+// The margin is one value per ray and BVH.  It costs the 1080p mesh 1.5 % (60.3
+// -> 61.2 ms), 3,000,001 ray queries 3.8 % (3.16 -> 3.28 ms); following the
+// distance to each node it cost 2.6 and 4.7 %.
 //
 // Conservative boxes.  With S = 2^15 cell inv and O' = (p - o) inv - S a
 // plane q lies at fma(1 + q 2^-15, S, O'), and 1 + q 2^-15 is q's byte put
@@ -48,7 +72,7 @@ namespace wf {
 // and one per level of the BLAS (each at most kMaxBvhDepth = 60 deep), and
 // the TLAS leaves left when an instance is entered.
 constexpr int kLaneStack = 128;
-constexpr float kSlack = 1.0f + 1.0f / 32768.0f;
+constexpr float kSlack = kWideSlack;
 constexpr float kNear = 1.0f + 1.0f / 131072.0f;
 
 // The ray of the current BVH as the node test wants it.
@@ -56,6 +80,7 @@ struct WideRay {
     V3 o, d;
     V3 inv;         // 1 / d, at most kInverseMax in size
     uint32_t oct4;  // per byte: bit a set when inv's component a is positive
+    float margin;   // how far outside its box a primitive's distance may lie
 };
 constexpr float kInverseMax = 1.2379400392853803e27f;  // 2^90
 
@@ -91,14 +116,25 @@ WF_DEV float plane(uint32_t w) {
 
 struct WideSlabs {
     float sx, sy, sz, ox, oy, oz, cull;
+    float nx, ny, nz;  // ox, oy, oz for the near planes, moved out by the margin
 };
+
+// WideRay::margin in a BVH with root box lo, hi.
+WF_DEV float cull_margin(V3 o, V3 lo, V3 hi, float reach, float base) {
+    float x = fmaxf(fabsf(lo.x - o.x), fabsf(hi.x - o.x)), y = fmaxf(fabsf(lo.y - o.y), fabsf(hi.y - o.y)),
+          z = fmaxf(fabsf(lo.z - o.z), fabsf(hi.z - o.z));
+    return __fmaf_rn(fmaxf(x, fmaxf(y, z)), reach, base);
+}
+WF_DEV float cull_margin(V3 o, const Box& b, float reach, float base) {
+    return cull_margin(o, V3{b.lo[0], b.lo[1], b.lo[2]}, V3{b.hi[0], b.hi[1], b.hi[2]}, reach, base);
+}
 
 template <int kByte>
 WF_DEV bool wide_child(const WideSlabs& b, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t fx, uint32_t fy,
                        uint32_t fz) {
-    float tx0 = __fmaf_rn(plane<kByte>(nx), b.sx, b.ox), tx1 = __fmaf_rn(plane<kByte>(fx), b.sx, b.ox);
-    float ty0 = __fmaf_rn(plane<kByte>(ny), b.sy, b.oy), ty1 = __fmaf_rn(plane<kByte>(fy), b.sy, b.oy);
-    float tz0 = __fmaf_rn(plane<kByte>(nz), b.sz, b.oz), tz1 = __fmaf_rn(plane<kByte>(fz), b.sz, b.oz);
+    float tx0 = __fmaf_rn(plane<kByte>(nx), b.sx, b.nx), tx1 = __fmaf_rn(plane<kByte>(fx), b.sx, b.ox);
+    float ty0 = __fmaf_rn(plane<kByte>(ny), b.sy, b.ny), ty1 = __fmaf_rn(plane<kByte>(fy), b.sy, b.oy);
+    float tz0 = __fmaf_rn(plane<kByte>(nz), b.sz, b.nz), tz1 = __fmaf_rn(plane<kByte>(fz), b.sz, b.oz);
     float entry = fmaxf(fmaxf(tx0, ty0), fmaxf(tz0, 0.0f));
     float exit = fminf(fminf(fminf(tx1, ty1), tz1) * kSlack, b.cull);
     return entry <= exit;
@@ -106,8 +142,10 @@ WF_DEV bool wide_child(const WideSlabs& b, uint32_t nx, uint32_t ny, uint32_t nz
 
 // Tests the children of wide node `index`: the internal hits (in visit
 // order: highest bit first) with the internal mask into `group`, the leaf
-// hits into `leaves`.
-WF_DEV void wide_node(const WideNode* nodes, uint32_t index, const WideRay& r, float closest_t, uint2& group,
+// hits into `leaves`.  Children whose entry is past `cull` are left out; for
+// a closest hit it is the entry of their boxes grown by the ray's margin.
+template <bool kAny>
+WF_DEV void wide_node(const WideNode* nodes, uint32_t index, const WideRay& r, float cull, uint2& group,
                       uint2& leaves) {
     const uint4* n = reinterpret_cast<const uint4*>(nodes + index);
     uint4 a = __ldg(n), b = __ldg(n + 1), c0 = __ldg(n + 2), c1 = __ldg(n + 3), c2 = __ldg(n + 4);
@@ -118,7 +156,10 @@ WF_DEV void wide_node(const WideNode* nodes, uint32_t index, const WideRay& r, f
     s.ox = __fmaf_rn(__uint_as_float(a.x) - r.o.x, r.inv.x, -s.sx);
     s.oy = __fmaf_rn(__uint_as_float(a.y) - r.o.y, r.inv.y, -s.sy);
     s.oz = __fmaf_rn(__uint_as_float(a.z) - r.o.z, r.inv.z, -s.sz);
-    s.cull = closest_t * kSlack;
+    s.nx = kAny ? s.ox : s.ox - fabsf(r.margin * r.inv.x);
+    s.ny = kAny ? s.oy : s.oy - fabsf(r.margin * r.inv.y);
+    s.nz = kAny ? s.oz : s.oz - fabsf(r.margin * r.inv.z);
+    s.cull = cull;
     bool px = r.oct4 & 1u, py = r.oct4 & 2u, pz = r.oct4 & 4u;
     uint32_t hits = 0;
 #pragma unroll
@@ -172,8 +213,8 @@ WF_DEV bool intersect_edges(V3 o, V3 d, V3 v0, V3 e1, V3 e2, float& t, float& u,
     return t > kRayMinDistance;
 }
 
-// Whether the BVH2's own box of a triangle passes its slab test; `entry` is
-// the box's entry distance.
+// Whether the BVH2's own box of a triangle (its vertices' bounds) passes its
+// slab test; `entry` is the box's entry distance.
 WF_DEV bool exact_triangle_box(const DeviceScene& s, uint32_t ti, const WideRay& r, float closest_t, float& entry) {
     TriVerts t = load_triangle(s, ti);
     return slab(r.o, exact_inverse(r), fminf(fminf(t.v0.x, t.v1.x), t.v2.x), fmaxf(fmaxf(t.v0.x, t.v1.x), t.v2.x),
@@ -182,6 +223,11 @@ WF_DEV bool exact_triangle_box(const DeviceScene& s, uint32_t ti, const WideRay&
 }
 WF_DEV bool exact_leaf_box(float4 lo, float4 hi, const WideRay& r, float closest_t, float& entry) {
     return slab(r.o, exact_inverse(r), lo.x, hi.x, lo.y, hi.y, lo.z, hi.z, closest_t, entry);
+}
+// Whether a box with entry distance `entry`, grown by the ray's margin, starts
+// past `cull` for certain (the margin moves no axis further than this).
+WF_DEV bool box_past(float entry, const WideRay& r, float cull) {
+    return entry > __fmaf_rn(r.margin, fmaxf(fabsf(r.inv.x), fmaxf(fabsf(r.inv.y), fabsf(r.inv.z))), cull);
 }
 
 // (By value: a lane's fields whose address is taken would live in memory.)
@@ -248,12 +294,12 @@ struct Lane {
     uint32_t state; // stage and the flags below
     uint32_t leaf;  // TLAS leaf entry of the current BLAS
     int size;       // stack entries
-    float4 world[3];  // world ray: (o, inv.x) (d, inv.y) (inv.z, oct4)
+    float4 world[3];  // world ray: (o, inv.x) (d, inv.y) (inv.z, oct4, margin, entry of the TLAS leaf)
     uint2 stack[kLaneStack];
 };
 enum : uint32_t {
     kStageTlas = 0, kStageBlas = 1, kStageDirect = 2, kStageDone = 3, kStageMask = 3,
-    kTie = 4,   // a candidate near the closest one was met
+    kTie = 4,   // the visit order could decide: a candidate, or the closest one's entry, is near the closest one
     kRedo = 8,  // the BVH2s must decide whatever comes
     kHit = 16   // kAny: occluded
 };
@@ -286,11 +332,24 @@ struct NoSink {
     WF_DEV void hit(float, float, float, uint32_t, uint32_t) {}
 };
 
-// The distance a box or candidate must start before: the ray's length, or
-// the closest hit with room for near ties.
+// The distance that a box's own test compares with: the ray's length, or none
+// (a closest hit's order is for lane_near to judge).
 template <bool kAny>
-WF_DEV float lane_limit(const Lane& L) {
-    return kAny ? L.t : L.t * kNear;
+WF_DEV float box_limit(const Lane& L) {
+    return kAny ? L.t : 1.0e30f;
+}
+
+// A closest-hit candidate at distance t <= L.t * kNear whose boxes start at
+// `entry`: returns whether it is the closest one so far, and notes whether
+// the order could matter.
+WF_DEV bool lane_near(Lane& L, float t, float entry) {
+    if (t >= L.t) {
+        L.state |= kTie;
+        return false;
+    }
+    if (t * kNear >= L.t || entry > t * kNear) L.state |= kTie; else L.state &= ~kTie;
+    L.t = t;
+    return true;
 }
 
 // Starts the TLAS or the direct list's BVH (each the only tree over its kind
@@ -310,7 +369,7 @@ WF_DEV void lane_occluded(Lane& L) { L.state |= kHit | kStageDone; }
 WF_DEV void lane_save_world(Lane& L) {
     L.world[0] = make_float4(L.r.o.x, L.r.o.y, L.r.o.z, L.r.inv.x);
     L.world[1] = make_float4(L.r.d.x, L.r.d.y, L.r.d.z, L.r.inv.y);
-    L.world[2] = make_float4(L.r.inv.z, __uint_as_float(L.r.oct4), 0.0f, 0.0f);
+    L.world[2] = make_float4(L.r.inv.z, __uint_as_float(L.r.oct4), L.r.margin, 0.0f);
 }
 WF_DEV void lane_restore_world(Lane& L) {
     float4 a = L.world[0], b = L.world[1], c = L.world[2];
@@ -318,9 +377,10 @@ WF_DEV void lane_restore_world(Lane& L) {
     L.r.d = f4xyz(b);
     L.r.inv = V3{a.w, b.w, c.x};
     L.r.oct4 = __float_as_uint(c.y);
+    L.r.margin = c.z;
 }
 
-// A triangle of the current BVH hit at distance t before lane_limit.
+// A triangle of the current BVH hit at distance t.
 template <bool kAny, typename Tally, typename Sink>
 WF_DEV void lane_candidate(Lane& L, const DeviceScene& s, Sink& sink, uint32_t ti, uint32_t material, float t, float u,
                            float v) {
@@ -333,20 +393,15 @@ WF_DEV void lane_candidate(Lane& L, const DeviceScene& s, Sink& sink, uint32_t t
         if (alpha_rejects<Tally>(s, material, ti, u, v)) return;
     }
     float entry;
-    if (!exact_triangle_box(s, ti, L.r, kAny ? L.t : 1.0e30f, entry)) return;
+    if (!exact_triangle_box(s, ti, L.r, box_limit<kAny>(L), entry)) return;
     if (kAny) {
         lane_occluded(L);
         return;
     }
-    if (entry > t * kNear) L.state |= kRedo;
-    if (t < L.t) {
-        if (t * kNear >= L.t) L.state |= kTie; else L.state &= ~kTie;
-        L.t = t;
-        uint32_t inst = blas ? __float_as_uint(__ldg(&s.wide.leaves[L.leaf].lo.w)) : kInvalid;
-        sink.hit(t, u, v, make_prim(blas ? kHitMesh : kHitTriangle, ti), inst);
-    } else {
-        L.state |= kTie;
-    }
+    if (blas) entry = fmaxf(entry, L.world[2].w);
+    if (!lane_near(L, t, entry)) return;
+    uint32_t inst = blas ? __float_as_uint(__ldg(&s.wide.leaves[L.leaf].lo.w)) : kInvalid;
+    sink.hit(t, u, v, make_prim(blas ? kHitMesh : kHitTriangle, ti), inst);
 }
 
 // Direct triangle list (last stage of traceRay / isOccluded): the lane
@@ -356,7 +411,8 @@ WF_DEV void lane_begin_direct(Lane& L, const DeviceScene& s) {
     lane_stage(L, kStageDone);
     if (s.direct_count == 0 || s.direct_bvh.root == kNoRoot) return;
     float near_t;
-    if (!slab_box(L.r.o, exact_inverse(L.r), s.direct_bvh.box, lane_limit<kAny>(L), near_t)) return;
+    if (!slab_box(L.r.o, exact_inverse(L.r), s.direct_bvh.box, box_limit<kAny>(L), near_t)) return;
+    if (!kAny) L.r.margin = cull_margin(L.r.o, s.direct_bvh.box, kWideReach, 0.0f);
     lane_stage(L, kStageDirect);
     lane_root(L, s.direct_bvh);
 }
@@ -391,6 +447,8 @@ WF_DEV void lane_begin(Lane& L, const DeviceScene& s, Sink& sink, V3 o, V3 d, fl
         sink.hit(h.t, h.u, h.v, h.prim, h.inst);
     }
     bool covered = wide_ray(L.r, o, d);
+    // (the TLAS's; lane_begin_direct has its own BVH's)
+    if (!kAny) L.r.margin = cull_margin(o, s.tlas.box, s.wide.reach, s.wide.base);
     lane_save_world(L);
     if (!covered || !s.wide.usable) {
         L.state |= kRedo;
@@ -398,7 +456,7 @@ WF_DEV void lane_begin(Lane& L, const DeviceScene& s, Sink& sink, V3 o, V3 d, fl
     }
     if (s.tlas.root != kNoRoot) {
         float near_t;
-        if (slab_box(o, exact_inverse(L.r), s.tlas.box, lane_limit<kAny>(L), near_t)) {
+        if (slab_box(o, exact_inverse(L.r), s.tlas.box, box_limit<kAny>(L), near_t)) {
             lane_stage(L, kStageTlas);
             lane_root(L, s.tlas);
             return;
@@ -432,9 +490,8 @@ WF_DEV void lane_tlas_leaf(Lane& L, const DeviceScene& s, Sink& sink, uint32_t e
     const float4* rec = reinterpret_cast<const float4*>(s.wide.leaves + entry);
     float4 lo = __ldg(rec + 3), hi = __ldg(rec + 4), x = __ldg(rec);
     uint32_t word = __float_as_uint(lo.w);
-    float limit = lane_limit<kAny>(L);
     float near_t;
-    if (!exact_leaf_box(lo, hi, L.r, limit, near_t)) return;
+    if (!exact_leaf_box(lo, hi, L.r, box_limit<kAny>(L), near_t)) return;
     if (word & 0x80000000u) {
         float t;
         tally.sphere();
@@ -443,15 +500,12 @@ WF_DEV void lane_tlas_leaf(Lane& L, const DeviceScene& s, Sink& sink, uint32_t e
             if (t < L.t) lane_occluded(L);
             return;
         }
-        if (t > limit) return;
-        if (near_t > t * kNear) L.state |= kRedo;
-        // equal distances among spheres go by their index: the BVH2s' turn
-        if (t * kNear >= L.t) L.state |= kTie; else L.state &= ~kTie;
-        if (t >= L.t) return;
-        L.t = t;
-        sink.hit(t, 0.0f, 0.0f, make_prim(kHitSphere, word & 0x7fffffffu), kInvalid);
+        // (equal distances among spheres go by their index: a tie too)
+        if (t <= L.t * kNear && lane_near(L, t, near_t))
+            sink.hit(t, 0.0f, 0.0f, make_prim(kHitSphere, word & 0x7fffffffu), kInvalid);
         return;
     }
+    if (!kAny && box_past(near_t, L.r, L.t * kSlack)) return;
     tally.instance();
     Instance in;
     in.w2l_x = x;
@@ -464,11 +518,15 @@ WF_DEV void lane_tlas_leaf(Lane& L, const DeviceScene& s, Sink& sink, uint32_t e
         return;
     }
     bool covered = wide_ray(L.r, to_local_vector(in, L.r.o - instance_translation(in)), to_local_vector(in, L.r.d));
-    if (!covered || !exact_leaf_box(root_lo, root_hi, L.r, limit, near_t)) {
+    if (!kAny) L.r.margin = cull_margin(L.r.o, f4xyz(root_lo), f4xyz(root_hi), kWideReach, 0.0f);
+    float local_t;
+    if (!covered || !exact_leaf_box(root_lo, root_hi, L.r, box_limit<kAny>(L), local_t) ||
+        (!kAny && box_past(local_t, L.r, L.t * kSlack))) {
         if (!covered) L.state |= kRedo;  // a scale the wide test's bounds do not cover
         lane_restore_world(L);
         return;
     }
+    if (!kAny) L.world[2].w = near_t;
     // what is left of this TLAS node waits below the BLAS's groups, under a mark
     if (L.group.y & 0xff000000u) L.stack[L.size++] = L.group;
     if (L.leaves.y) L.stack[L.size++] = L.leaves;
@@ -489,7 +547,8 @@ WF_DEV void lane_node(Lane& L, const DeviceScene& s, Tally& tally) {
         uint32_t node = wide_next(rest, L.r.oct4);
         if (rest.y & 0xff000000u) L.stack[L.size++] = rest;
         tally.node();
-        wide_node(s.wide.nodes, node, L.r, L.t, L.group, L.leaves);
+        float slack = !kAny && (L.state & kStageMask) == kStageTlas ? s.wide.slack : kSlack;
+        wide_node<kAny>(s.wide.nodes, node, L.r, L.t * slack, L.group, L.leaves);
     }
 }
 

@@ -54,8 +54,10 @@ __global__ void k_wide_emit(DeviceScene s, const BvhRef* roots, uint32_t count, 
 
 cudaError_t build_wide_bvh(DeviceScene& view, const std::vector<BvhRef>& roots, uint32_t node_count,
                            uint32_t tlas_root, std::vector<void*>& allocations, uint64_t& bytes) {
-    view.wide = WideBvh{};
-    if (roots.empty()) return cudaSuccess;
+    if (roots.empty()) {
+        view.wide.usable = 0u;
+        return cudaSuccess;
+    }
     uint32_t root_count = uint32_t(roots.size());
     // Wide nodes other than the roots stand for distinct internal BVH2 nodes.
     size_t capacity = size_t(node_count) + root_count;
@@ -109,7 +111,12 @@ cudaError_t build_wide_bvh(DeviceScene& view, const std::vector<BvhRef>& roots, 
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     cudaFree(scratch);
-    if (e == cudaSuccess) view.wide = WideBvh{nodes, triangles, leaves, host[3] ? 0u : 1u};
+    if (e == cudaSuccess) {
+        view.wide.nodes = nodes;
+        view.wide.triangles = triangles;
+        view.wide.leaves = leaves;
+        if (host[3]) view.wide.usable = 0u;
+    }
     return e;
 }
 

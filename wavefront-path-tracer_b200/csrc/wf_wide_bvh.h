@@ -7,7 +7,7 @@ namespace wf {
 
 // Collapses every BVH2 of the scene (BLASes, TLAS, direct list), whose nodes,
 // triangles, instances and BLAS records are already on the device, into
-// 8-wide compressed nodes and fills in view.wide.  Tree i (roots[i], with its
+// 8-wide compressed nodes and completes view.wide (HostScene::margins).  Tree i (roots[i], with its
 // root box) gets wide node i as its root; tree `tlas_root` is the TLAS
 // (kNoWide: none).  `node_count` is the number of BVH2 nodes.  The arrays go
 // to `allocations` and their size is added to `bytes`.  Runs on the legacy
