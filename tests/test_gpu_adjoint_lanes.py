@@ -44,3 +44,37 @@ def test_samples_average(cuda, spp, depth, size):
     assert np.linalg.norm(want) > 0
     assert np.linalg.norm(grads - want) <= 1e-4 * np.linalg.norm(want)
     dev.close()
+
+
+@pytest.mark.parametrize("spp,pixels", [(1, 32), (1, 7), (8, 4), (3, 10), (32, 2)])
+def test_pixels_meet_in_double(cuda, spp, pixels):
+    """Gradients are sums of float terms of the single pixels, added in
+    double.  A pixel's terms do not depend on the other pixels' adjoints, so
+    the gradient of a large adjoint (2^24) at one pixel and small ones at its
+    neighbours in the warp is the sum of the two gradients.  In double the
+    sums lose at most spp x pixels x depth = 128 times 2^-53 of the large
+    terms, which may be some 2^6 of their sum: 2^-40 of it.  A float sum across
+    pixels would lose 2^-24 of it, as much as the small ones' terms are.
+    Samples of one pixel always have the same adjoint here, so how they meet
+    is not what is tested."""
+    torch = cuda
+    scene, cam, n, _ = scenes.cornell_inverse(256, 256, cells=1)  # few large triangles: one for many lanes
+    a, r = (torch.from_numpy(x).cuda() for x in scenes.inverse_parameters(scene, n, seed=9))
+    dev = wfpt.DeviceScene(scene)
+    depth = 4
+    cfg = diff.diff_config(256, 256, spp, depth, n, sample_start=5, crop=(100, 200, pixels, 1))
+    small = torch.zeros(256, 256, 3, device="cuda")
+    small[200, 100:100 + pixels] = 1.0
+    small[200, 100] = 0.0
+    large = torch.zeros(256, 256, 3, device="cuda")
+    large[200, 100] = 2.0 ** 24
+
+    def gradient(adjoint):
+        return np.concatenate([x.double().cpu().numpy().ravel()
+                               for x in diff.backward(dev, cam, cfg, a, r, 1.0, adjoint)])
+
+    g_small, g_large, g_both = gradient(small), gradient(large), gradient(small + large)
+    bound = 2.0 ** -40 * np.abs(g_large).max()
+    assert np.abs(g_small).max() > 1e3 * bound
+    assert np.abs(g_both - (g_large + g_small)).max() <= bound
+    dev.close()

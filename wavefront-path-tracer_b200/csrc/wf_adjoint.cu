@@ -109,26 +109,27 @@ WF_DEV uint32_t parameter_index(const DeviceScene& s, uint32_t prim) {
 }
 
 // Gradient contributions of one vertex, summed over the lanes of a warp
-// that hit the same triangle (all 32 lanes call this together).  One lane
-// per triangle adds the sums with double atomics.
+// that hit the same triangle (all 32 lanes call this together): one lane per
+// triangle adds them up in double and makes the double atomics, so terms of
+// different pixels never meet in float (the lanes are of up to 32 pixels).
 WF_DEV void flush_vertex(uint32_t key, float4 value, float4* warp_buffer, const DiffGrads& G) {
     uint32_t lane = threadIdx.x & 31;
     unsigned peers = __match_any_sync(0xffffffffu, key);
     warp_buffer[lane] = value;
     __syncwarp();
     if (key != kInvalid && lane == uint32_t(__ffs(peers) - 1)) {
-        float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        double x = 0.0, y = 0.0, z = 0.0, w = 0.0;
         for (unsigned m = peers; m; m &= m - 1) {
             float4 v = warp_buffer[__ffs(m) - 1];
-            sum.x += v.x;
-            sum.y += v.y;
-            sum.z += v.z;
-            sum.w += v.w;
+            x += double(v.x);
+            y += double(v.y);
+            z += double(v.z);
+            w += double(v.w);
         }
-        if (sum.x != 0.0f) atomicAdd(&G.albedo[3 * key], double(sum.x));
-        if (sum.y != 0.0f) atomicAdd(&G.albedo[3 * key + 1], double(sum.y));
-        if (sum.z != 0.0f) atomicAdd(&G.albedo[3 * key + 2], double(sum.z));
-        if (sum.w != 0.0f) atomicAdd(&G.roughness[key], double(sum.w));
+        if (x != 0.0) atomicAdd(&G.albedo[3 * key], x);
+        if (y != 0.0) atomicAdd(&G.albedo[3 * key + 1], y);
+        if (z != 0.0) atomicAdd(&G.albedo[3 * key + 2], z);
+        if (w != 0.0) atomicAdd(&G.roughness[key], w);
     }
     __syncwarp();
 }
