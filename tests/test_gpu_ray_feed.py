@@ -22,6 +22,12 @@ def _scene(which, w, h):
         return scenes.sphere_field(w, h, frequency=8, seed=5)
     if which == "room":  # alpha-masked textures
         return scenes.textured_room(w, h)
+    if which == "masked lists":  # both: the fully generic kernels
+        scene, cam = scenes.textured_room(w, h)
+        lamp = scene.add_material(wfpt.material(abi.MAT_EMISSIVE, (1, 1, 1), (8, 8, 8)))
+        scene.material_textures = np.concatenate([scene.material_textures, scenes.material_textures()])
+        scene.static_triangles = scenes.quad((-.2, .9, -.2), (.2, .9, -.2), (.2, .9, .2), (-.2, .9, .2), lamp)
+        return scene, cam
     if which == "contact":  # glass cubes on an instanced floor, seen from among them: faces on one plane
         scene = wfpt.Scene()
         rng = np.random.default_rng(5)
@@ -34,13 +40,13 @@ def _scene(which, w, h):
              for k, (x, z) in enumerate(rng.uniform(-6, 6, (60, 2)))])
         return scene, scenes.look_at_camera((0.494, 0.02, 6.4), (0.45, -0.3, 6.2), 90.0, w, h)
     scene, cam = scenes.cornell_box(w, h)
-    if which == "lists":  # primitives outside the BVHs: the generic kernels
+    if which == "lists":  # primitives outside the BVHs
         scene.static_triangles = scenes.quad((-1, 0, 1), (1, 0, 1), (1, 0.5, 1), (-1, 0.5, 1), 1)
         scene.triangles = scenes.quad((-1, 1, 1), (0, 1, 1), (0, 2, 0.5), (-1, 2, 0.5), 2)
     return scene, cam
 
 
-@pytest.mark.parametrize("which", ["cornell", "mesh", "spheres", "room", "lists", "contact"])
+@pytest.mark.parametrize("which", ["cornell", "mesh", "spheres", "room", "lists", "masked lists", "contact"])
 @pytest.mark.parametrize("size", [(1, 1), (3, 5), (65, 33), (257, 129)])
 def test_frame_does_not_depend_on_launch_size(cuda, which, size):
     w, h = size
@@ -74,7 +80,7 @@ def test_more_rays_than_lanes(cuda):
     assert np.array_equal(images[0].view(np.uint32), images[1].view(np.uint32))
 
 
-@pytest.mark.parametrize("which", ["mesh", "room", "lists"])
+@pytest.mark.parametrize("which", ["mesh", "room", "lists", "masked lists"])
 def test_large_ray_batches_match_small_ones(cuda, which):
     """Batches around the size from which lanes are refilled (8 CTAs of 128 on
     each SM, twice) against the same rays in small ones, record for record."""

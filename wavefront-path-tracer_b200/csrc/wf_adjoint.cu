@@ -166,8 +166,7 @@ WF_HDI DiffLanes diff_lanes(uint32_t spp) {
 // delta * dU/dtheta to the gradients and returns the replayed radiance.  In
 // adjoint mode all 32 lanes of the warp call it together (`alive` false for
 // lanes without a path) and run the same number of vertex steps.
-// Tally: the traversal variant (Opaque<NoTally> for scenes that allow it,
-// wf_scene::opaque).
+// Tally: the scene's traversal variant (with_variant).
 // kRecord: the non-adjoint replay fills `record`, the adjoint one reads it.
 template <bool kAdjoint, bool kRecord, typename Tally>
 WF_DEV V3 diff_path(const DeviceScene& s, const DiffParams& P, const DiffSettings& cfg, uint32_t px, uint32_t py,
@@ -463,10 +462,9 @@ extern "C" wf_status wf_diff_forward(const wf_scene* scene, const wf_camera* cam
     cudaError_t ce = cudaMemsetAsync(error, 0, sizeof(uint32_t), st);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync");
     DiffParams P{albedo, roughness, emission_scale};
-    if (!scene->opaque())
-        k_diff_forward<NoTally><<<diff_grid(cfg), 128, 0, st>>>(scene->view, P, cfg, image, error);
-    else
-        k_diff_forward<Opaque<NoTally>><<<diff_grid(cfg), 128, 0, st>>>(scene->view, P, cfg, image, error);
+    with_variant<NoTally>(scene->opaque(), scene->listless(), [&](auto tally) {
+        k_diff_forward<decltype(tally)><<<diff_grid(cfg), 128, 0, st>>>(scene->view, P, cfg, image, error);
+    });
     ce = cudaGetLastError();
     if (ce != cudaSuccess) return cuda_fail(ce, "k_diff_forward");
     return diff_finish(error, st);
@@ -487,10 +485,9 @@ extern "C" wf_status wf_diff_backward(const wf_scene* scene, const wf_camera* ca
     DiffParams P{albedo, roughness, emission_scale};
     DiffGrads G{d_albedo, d_roughness, d_emission_scale};
     uint32_t blocks = diff_grid(cfg);
-    if (!scene->opaque())
-        k_diff_backward<NoTally><<<blocks, 128, 0, st>>>(scene->view, P, cfg, d_image, G, error);
-    else
-        k_diff_backward<Opaque<NoTally>><<<blocks, 128, 0, st>>>(scene->view, P, cfg, d_image, G, error);
+    with_variant<NoTally>(scene->opaque(), scene->listless(), [&](auto tally) {
+        k_diff_backward<decltype(tally)><<<blocks, 128, 0, st>>>(scene->view, P, cfg, d_image, G, error);
+    });
     ce = cudaGetLastError();
     if (ce != cudaSuccess) return cuda_fail(ce, "k_diff_backward");
     return diff_finish(error, st);

@@ -55,7 +55,8 @@ struct BatchView {
 struct wf_batch {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
-    bool opaque = true;     // every job's scene is (wf_scene::opaque): the Opaque<> trace and shadow kernels
+    bool opaque = true;     // every job's scene is (wf_scene::opaque, ::listless): which
+    bool listless = true;   // variant of the trace and shadow kernels (with_variant)
     bool textured = false;  // some job's scene has textured materials: k_batch_shade<true>
     bool direct = true;     // every job's scene is eventless (wf_scene::eventless): k_batch_shade_direct
     int device = 0, sm_count = 148;
@@ -509,12 +510,10 @@ wf_status capture_batch(wf_batch* b) {
         uint32_t nxt = cur ^ 1;
         uint32_t* cur_count = &b->counters->queue_count[cur];
         uint32_t* next_count = &b->counters->queue_count[nxt];
-        if (b->opaque)
-            k_batch_trace<Opaque<NoTally>><<<batch_grid(b, 0, cap, b->block), b->block, 0, st>>>(
+        with_variant<NoTally>(b->opaque, b->listless, [&](auto tally) {
+            k_batch_trace<decltype(tally)><<<batch_grid(b, 0, cap, b->block), b->block, 0, st>>>(
                 b->view, b->paths, b->queue[cur], cur_count, b->hit_a, b->hit_inst, b->counters, b->refill);
-        else
-            k_batch_trace<NoTally><<<batch_grid(b, 0, cap, b->block), b->block, 0, st>>>(
-                b->view, b->paths, b->queue[cur], cur_count, b->hit_a, b->hit_inst, b->counters, b->refill);
+        });
         if (b->direct) {
             if (b->textured)
                 k_batch_shade_direct<true><<<batch_grid(b, 1, cap, 128), 128, 0, st>>>(
@@ -534,14 +533,11 @@ wf_status capture_batch(wf_batch* b) {
             k_batch_shade<false><<<batch_grid(b, 1, cap, 128), 128, 0, st>>>(
                 b->view, b->paths, b->queue[cur], cur_count, b->hit_a, b->hit_inst, b->terms, b->shade_out,
                 b->shadow_origin, b->shadow_dir, b->shadow_capacity, b->counters, next_count);
-        if (b->opaque)
-            k_batch_shadow<Opaque<NoTally>><<<batch_grid(b, 2, b->shadow_capacity, b->block), b->block, 0, st>>>(
-                b->view, b->shadow_origin, b->shadow_dir, b->shadow_result, b->shadow_chain, b->counters, b->shadow_capacity,
-                b->refill);
-        else
-            k_batch_shadow<NoTally><<<batch_grid(b, 2, b->shadow_capacity, b->block), b->block, 0, st>>>(
-                b->view, b->shadow_origin, b->shadow_dir, b->shadow_result, b->shadow_chain, b->counters, b->shadow_capacity,
-                b->refill);
+        with_variant<NoTally>(b->opaque, b->listless, [&](auto tally) {
+            k_batch_shadow<decltype(tally)><<<batch_grid(b, 2, b->shadow_capacity, b->block), b->block, 0, st>>>(
+                b->view, b->shadow_origin, b->shadow_dir, b->shadow_result, b->shadow_chain, b->counters,
+                b->shadow_capacity, b->refill);
+        });
         k_batch_finalize<<<batch_grid(b, 3, cap, 256), 256, 0, st>>>(
             b->view, b->paths, b->queue[cur], cur_count, b->terms, b->shade_out, b->shadow_result, b->queue[nxt],
             next_count, cap, b->counters);
@@ -617,6 +613,7 @@ wf_status batch_create(const wf_batch_job* jobs, uint32_t count, const wf_batch_
     b->refill = config.refill_threshold ? config.refill_threshold : 8u;
     for (uint32_t i = 0; i < count; ++i) {
         b->opaque = b->opaque && jobs[i].scene->opaque();
+        b->listless = b->listless && jobs[i].scene->listless();
         b->textured = b->textured || jobs[i].scene->textured;
         b->direct = b->direct && jobs[i].scene->eventless();
     }
@@ -715,16 +712,18 @@ wf_status batch_create(const wf_batch_job* jobs, uint32_t count, const wf_batch_
     b->view.job_count = count;
     b->view.units = b->units;
     b->view.pixels = uint32_t(pixels_total);
-    WF_BATCH_CUDA(b->opaque ? batch_resident(bp, 0, k_batch_trace<Opaque<NoTally>>, b->block)
-                            : batch_resident(bp, 0, k_batch_trace<NoTally>, b->block));
+    WF_BATCH_CUDA(with_variant<NoTally>(b->opaque, b->listless, [&](auto tally) {
+        return batch_resident(bp, 0, k_batch_trace<decltype(tally)>, b->block);
+    }));
     if (b->direct)
         WF_BATCH_CUDA(b->textured ? batch_resident(bp, 1, k_batch_shade_direct<true>, 128)
                                   : batch_resident(bp, 1, k_batch_shade_direct<false>, 128));
     else
         WF_BATCH_CUDA(b->textured ? batch_resident(bp, 1, k_batch_shade<true>, 128)
                                   : batch_resident(bp, 1, k_batch_shade<false>, 128));
-    WF_BATCH_CUDA(b->opaque ? batch_resident(bp, 2, k_batch_shadow<Opaque<NoTally>>, b->block)
-                            : batch_resident(bp, 2, k_batch_shadow<NoTally>, b->block));
+    WF_BATCH_CUDA(with_variant<NoTally>(b->opaque, b->listless, [&](auto tally) {
+        return batch_resident(bp, 2, k_batch_shadow<decltype(tally)>, b->block);
+    }));
     WF_BATCH_CUDA(batch_resident(bp, 3, k_batch_finalize, 256));
     if (wf_status e = capture_batch(bp)) {
         abandon_capture(b->stream);

@@ -98,13 +98,13 @@ struct wf_scene {
     uint32_t gpu_bvh_builds = 0;
     double bvh_build_ms = 0.0;
     bool alpha_textures = false;  // some material is alpha-masked with an albedo texture
-    // every primitive is in a BVH (direct spheres aside): the Listless<> kernels
+    // every primitive is in a BVH (direct spheres aside)
     bool listless() const {
         return view.direct_instance_count == 0 && view.static_count == 0 &&
                (view.direct_count == 0 || view.direct_bvh.root != wf::kNoRoot);
     }
-    // ... and no material is alpha-textured: the Opaque<> kernels
-    bool opaque() const { return !alpha_textures && listless(); }
+    // no material is alpha-textured
+    bool opaque() const { return !alpha_textures; }
     // nothing that shading samples with a shadow ray: no lights and no environment
     bool eventless() const { return view.light_count == 0 && view.punctual_count == 0 && !view.env.present; }
     bool textured = false;        // some material has a texture binding

@@ -801,11 +801,20 @@ __global__ void __launch_bounds__(128, 8) k_persistent(const __grid_constant__ D
 }
 
 // The persistent kernel for a scene: without the alpha test when no material
-// is alpha-textured, without the texture code when none is textured.
-const void* persistent_kernel(bool opaque, bool textured) {
-    if (!opaque) return reinterpret_cast<const void*>(k_persistent<NoTally, true>);
-    return textured ? reinterpret_cast<const void*>(k_persistent<Opaque<NoTally>, true>)
-                    : reinterpret_cast<const void*>(k_persistent<Opaque<NoTally>, false>);
+// is alpha-textured, then without the texture code when none is textured and
+// without the list scans when every primitive is in a BVH.
+constexpr int kPersistentVariants = 5;
+int persistent_variant(bool opaque, bool listless, bool textured) {
+    return !opaque ? 0 : 1 + (textured ? 1 : 0) + (listless ? 0 : 2);
+}
+const void* persistent_kernel(int variant) {
+    switch (variant) {
+        case 1: return reinterpret_cast<const void*>(k_persistent<Opaque<NoTally>, false>);
+        case 2: return reinterpret_cast<const void*>(k_persistent<Opaque<NoTally>, true>);
+        case 3: return reinterpret_cast<const void*>(k_persistent<Lists<NoTally>, false>);
+        case 4: return reinterpret_cast<const void*>(k_persistent<Lists<NoTally>, true>);
+        default: return reinterpret_cast<const void*>(k_persistent<NoTally, true>);
+    }
 }
 
 // The phased persistent kernel (WF_MODE_PERSISTENT renderers): one
@@ -923,11 +932,17 @@ __global__ void __launch_bounds__(128, WF_PHASED_CTAS) k_persistent_phased(const
     }
 }
 
-const void* phased_kernel(bool opaque, bool textured) {
-    if (!opaque) return reinterpret_cast<const void*>(k_persistent_phased<NoTally, true>);
-    return textured ? reinterpret_cast<const void*>(k_persistent_phased<Opaque<NoTally>, true>)
-                    : reinterpret_cast<const void*>(k_persistent_phased<Opaque<NoTally>, false>);
+const void* phased_kernel(int variant) {
+    switch (variant) {
+        case 1: return reinterpret_cast<const void*>(k_persistent_phased<Opaque<NoTally>, false>);
+        case 2: return reinterpret_cast<const void*>(k_persistent_phased<Opaque<NoTally>, true>);
+        case 3: return reinterpret_cast<const void*>(k_persistent_phased<Lists<NoTally>, false>);
+        case 4: return reinterpret_cast<const void*>(k_persistent_phased<Lists<NoTally>, true>);
+        default: return reinterpret_cast<const void*>(k_persistent_phased<NoTally, true>);
+    }
 }
+// The kernels of a renderer's scene.
+int persistent_variant(const wf_renderer* r) { return persistent_variant(r->opaque, r->listless, r->textured); }
 
 // ---------------------------------------------------------------- batch API
 // The record of a hit from the traversal's state.
@@ -1404,11 +1419,11 @@ wf_status build_photon_map(wf_renderer* r) {
     return WF_OK;
 }
 
-// k_trace / k_shadow for this renderer's scene: the Opaque<> variants (the
-// per-hit alpha-texture test and the linear primitive lists compiled out,
-// fewer registers) where the scene has neither (wf_scene::opaque), else the
-// Listless<> ones where it has no lists: the list scans' calls cost the loop
-// spills (960x540 textured room, 4 samples: 7.50 -> 6.95 ms).
+// k_trace / k_shadow for this renderer's scene: the per-hit alpha-texture
+// test and the scans of the linear primitive lists compiled out where the
+// scene has none (the list scans' calls cost the loop spills: 960x540 textured
+// room, 4 samples: 7.50 -> 6.95 ms).  Camera rays (trace_coherent) scan the
+// lists by their counts and have only the alpha variants.
 template <typename Tally, bool kLanes, typename... A>
 void launch_trace(const wf_renderer* r, uint32_t grid_size, uint32_t block, cudaStream_t st, A... args) {
     if constexpr (!kLanes) {
@@ -1416,12 +1431,10 @@ void launch_trace(const wf_renderer* r, uint32_t grid_size, uint32_t block, cuda
             k_trace_camera<Opaque<Tally>><<<grid_size, block, 0, st>>>(args...);
         else
             k_trace_camera<Tally><<<grid_size, block, 0, st>>>(args...);
-    } else if (r->opaque) {
-        k_trace<Opaque<Tally>, kLanes><<<grid_size, block, 0, st>>>(args...);
-    } else if (r->listless) {
-        k_trace<Listless<Tally>, kLanes><<<grid_size, block, 0, st>>>(args...);
     } else {
-        k_trace<Tally, kLanes><<<grid_size, block, 0, st>>>(args...);
+        with_variant<Tally>(r->opaque, r->listless, [&](auto tally) {
+            k_trace<decltype(tally), kLanes><<<grid_size, block, 0, st>>>(args...);
+        });
     }
 }
 // k_shade with the texture code only for scenes that have textured materials.
@@ -1441,12 +1454,9 @@ void launch_shade_direct(const wf_renderer* r, uint32_t grid_size, uint32_t bloc
 }
 template <typename Tally, typename... A>
 void launch_shadow(const wf_renderer* r, uint32_t grid_size, uint32_t block, cudaStream_t st, A... args) {
-    if (r->opaque)
-        k_shadow<Opaque<Tally>><<<grid_size, block, 0, st>>>(args...);
-    else if (r->listless)
-        k_shadow<Listless<Tally>><<<grid_size, block, 0, st>>>(args...);
-    else
-        k_shadow<Tally><<<grid_size, block, 0, st>>>(args...);
+    with_variant<Tally>(r->opaque, r->listless, [&](auto tally) {
+        k_shadow<decltype(tally)><<<grid_size, block, 0, st>>>(args...);
+    });
 }
 
 wf_status capture_graph(wf_renderer* r) {
@@ -1641,7 +1651,7 @@ cudaError_t launch_phased(wf_renderer* r, cudaStream_t st, uint64_t paths) {
     void* args[] = {&s, &rp, &tp, &c, &b};
     uint32_t blocks = persistent_grid(r->config.persistent_blocks, r->phased_blocks, r->sm_count,
                                       std::min<uint64_t>(paths, r->capacity));
-    return cudaLaunchCooperativeKernel(phased_kernel(r->opaque, r->textured), dim3(blocks),
+    return cudaLaunchCooperativeKernel(phased_kernel(persistent_variant(r)), dim3(blocks),
                                        dim3(r->persistent_block_size), args, 0, st);
 }
 
@@ -1663,7 +1673,7 @@ cudaError_t launch_fused(wf_renderer* r, cudaStream_t st, uint64_t paths) {
     void* args[] = {&s, &rp, &tp, &c, &ps, &q0, &q1, &cap, &fb, &chunk};
     uint32_t blocks = persistent_grid(r->config.persistent_blocks, r->persistent_blocks, r->sm_count,
                                       std::min<uint64_t>(paths, r->capacity));
-    return cudaLaunchCooperativeKernel(persistent_kernel(r->opaque, r->textured), dim3(blocks),
+    return cudaLaunchCooperativeKernel(persistent_kernel(persistent_variant(r)), dim3(blocks),
                                        dim3(r->persistent_block_size), args, 0, st);
 }
 
@@ -1843,16 +1853,16 @@ wf_status renderer_create_impl(const wf_scene* scene, const wf_camera* camera, c
         }
     }
     if (c.mode != WF_MODE_PERSISTENT) {
-        WF_CUDA(r->opaque     ? resident_grid(rr, 0, k_trace<Opaque<NoTally>>, r->block_trace)
-                : r->listless ? resident_grid(rr, 0, k_trace<Listless<NoTally>>, r->block_trace)
-                              : resident_grid(rr, 0, k_trace<NoTally>, r->block_trace));
+        WF_CUDA(with_variant<NoTally>(r->opaque, r->listless, [&](auto tally) {
+            return resident_grid(rr, 0, k_trace<decltype(tally)>, r->block_trace);
+        }));
         WF_CUDA(r->opaque ? resident_grid(rr, 5, k_trace_camera<Opaque<NoTally>>, r->block_camera)
                           : resident_grid(rr, 5, k_trace_camera<NoTally>, r->block_camera));
         WF_CUDA(r->textured ? resident_grid(rr, 1, k_shade<true>, r->block_shade)
                             : resident_grid(rr, 1, k_shade<false>, r->block_shade));
-        WF_CUDA(r->opaque     ? resident_grid(rr, 2, k_shadow<Opaque<NoTally>>, r->block_trace)
-                : r->listless ? resident_grid(rr, 2, k_shadow<Listless<NoTally>>, r->block_trace)
-                              : resident_grid(rr, 2, k_shadow<NoTally>, r->block_trace));
+        WF_CUDA(with_variant<NoTally>(r->opaque, r->listless, [&](auto tally) {
+            return resident_grid(rr, 2, k_shadow<decltype(tally)>, r->block_trace);
+        }));
         WF_CUDA(resident_grid(rr, 3, k_finalize<true>, r->block_finalize));
     } else {
         int cooperative = 0;
@@ -1862,10 +1872,10 @@ wf_status renderer_create_impl(const wf_scene* scene, const wf_camera* camera, c
             return fail(WF_ERR_INVALID_ARG, "unknown persistent kernel %u", c.persistent_stages);
         r->persistent_block_size = 128;
         int per_sm = 0;
-        WF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_kernel(r->opaque, r->textured),
+        WF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_kernel(persistent_variant(rr)),
                                                               int(r->persistent_block_size), 0));
         int phased_per_sm = 0;
-        WF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&phased_per_sm, phased_kernel(r->opaque, r->textured),
+        WF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&phased_per_sm, phased_kernel(persistent_variant(rr)),
                                                               int(r->persistent_block_size), 0));
         if (per_sm <= 0 || phased_per_sm <= 0) return fail(WF_ERR_UNSUPPORTED, "the persistent kernel cannot be resident");
         // the largest grids; persistent_grid picks each launch's
@@ -2291,15 +2301,14 @@ wf_status trace_closest_batch(const wf_scene* scene, const wf_ray* rays, uint32_
     if (count == 0) return WF_OK;
     uint32_t blocks = (count - 1) / 128 + 1;
     if (large_batch(scene, count)) {
-        if (scene->opaque())
-            k_trace_blocks<Opaque<NoTally>><<<batch_ctas(scene), 128, 0, stream>>>(scene->view, rays, count, hits);
-        else
-            k_trace_blocks<NoTally><<<batch_ctas(scene), 128, 0, stream>>>(scene->view, rays, count, hits);
+        with_variant<NoTally>(scene->opaque(), scene->listless(), [&](auto tally) {
+            k_trace_blocks<decltype(tally)><<<batch_ctas(scene), 128, 0, stream>>>(scene->view, rays, count, hits);
+        });
         k_finish_batch<<<blocks, 128, 0, stream>>>(scene->view, rays, count, hits);
-    } else if (scene->opaque()) {
-        k_trace_batch<Opaque<NoTally>><<<blocks, 128, 0, stream>>>(scene->view, rays, count, hits);
     } else {
-        k_trace_batch<NoTally><<<blocks, 128, 0, stream>>>(scene->view, rays, count, hits);
+        with_variant<NoTally>(scene->opaque(), scene->listless(), [&](auto tally) {
+            k_trace_batch<decltype(tally)><<<blocks, 128, 0, stream>>>(scene->view, rays, count, hits);
+        });
     }
     WF_CUDA(cudaGetLastError());
     return WF_OK;
@@ -2310,17 +2319,15 @@ wf_status trace_any_batch(const wf_scene* scene, const wf_ray* rays, const float
     if (count == 0) return WF_OK;
     uint32_t blocks = (count - 1) / 128 + 1;
     if (large_batch(scene, count)) {
-        if (scene->opaque())
-            k_any_blocks<Opaque<NoTally>>
+        with_variant<NoTally>(scene->opaque(), scene->listless(), [&](auto tally) {
+            k_any_blocks<decltype(tally)>
                 <<<batch_ctas(scene), 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
-        else
-            k_any_blocks<NoTally>
-                <<<batch_ctas(scene), 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
+        });
         k_any_settle<<<blocks, 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
-    } else if (scene->opaque()) {
-        k_any_batch<Opaque<NoTally>><<<blocks, 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
     } else {
-        k_any_batch<NoTally><<<blocks, 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
+        with_variant<NoTally>(scene->opaque(), scene->listless(), [&](auto tally) {
+            k_any_batch<decltype(tally)><<<blocks, 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
+        });
     }
     WF_CUDA(cudaGetLastError());
     return WF_OK;
@@ -2366,7 +2373,7 @@ constexpr int kStaticMaxDevices = 64;
 std::mutex g_static_mutex;
 unsigned char* g_static_base[kStaticMaxDevices] = {};
 unsigned long long g_static_context[kStaticMaxDevices] = {};  // context the address belongs to
-uint32_t g_static_resident[kStaticMaxDevices][3] = {};  // per persistent-kernel variant
+uint32_t g_static_resident[kStaticMaxDevices][kPersistentVariants] = {};  // per persistent-kernel variant
 
 // Unique id of the calling thread's current context (cuCtxGetId), or 0 when
 // none is current.  A device whose context is re-created (cudaDeviceReset,
@@ -2446,9 +2453,8 @@ extern "C" wf_status wf_render_tile_static(const wf_scene* scene, const wf_camer
     if (device < 0 || device >= kStaticMaxDevices) return fail(WF_ERR_UNSUPPORTED, "device index %d", device);
     unsigned char* base = nullptr;
     uint32_t resident = 0;
-    const bool opaque = scene->opaque();
-    const void* kernel = persistent_kernel(opaque, scene->textured);
-    const int variant = !opaque ? 0 : (scene->textured ? 1 : 2);
+    const int variant = persistent_variant(scene->opaque(), scene->listless(), scene->textured);
+    const void* kernel = persistent_kernel(variant);
     {
         std::lock_guard<std::mutex> lock(g_static_mutex);
         unsigned long long context = 0;

@@ -94,8 +94,8 @@ struct wf_renderer {
     wf::RenderParams params{};
     cudaStream_t stream = nullptr;
     bool own_stream = false;
-    bool opaque = true;     // wf_scene::opaque: the Opaque<> trace and shadow kernels
-    bool listless = true;   // wf_scene::listless: the Listless<> ones otherwise
+    bool opaque = true;     // wf_scene::opaque, ::listless: which variant of
+    bool listless = true;   // the traversing kernels (with_variant)
     bool direct = false;    // wf_scene::eventless and no photon map: k_shade_direct (graph mode)
     bool textured = false;  // some textured material: k_shade<true>
     bool sort_shading = true;  // material-sort the hits before shading (k_classify, k_scatter)

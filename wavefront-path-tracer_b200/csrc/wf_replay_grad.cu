@@ -199,18 +199,16 @@ extern "C" wf_status wf_render_albedo_gradient(wf_renderer* r, uint32_t x, uint3
     TileDev tile{x, y, width, height, 0};
     uint32_t pixels = width * height;
     uint32_t blocks = (pixels + 127) / 128;  // one pixel per thread; the hardware balances the CTAs
-    // The variants of the fused persistent kernel: the alpha test only when
-    // some material is alpha-textured, the texture code only when one is
-    // textured.
-    if (!r->opaque)
-        launch_gradient<NoTally, true>(blocks, st, s, r->params, tile, sample_start, sample_count, gp, adjoint, image,
-                                       gradient);
-    else if (r->textured)
-        launch_gradient<Opaque<NoTally>, true>(blocks, st, s, r->params, tile, sample_start, sample_count, gp,
-                                               adjoint, image, gradient);
-    else
-        launch_gradient<Opaque<NoTally>, false>(blocks, st, s, r->params, tile, sample_start, sample_count, gp,
-                                                adjoint, image, gradient);
+    // The variants of the fused persistent kernel (persistent_kernel).
+    with_variant<NoTally>(r->opaque, r->listless || !r->opaque, [&](auto tally) {
+        using Tally = std::conditional_t<decltype(tally)::kAlphaTextures, NoTally, decltype(tally)>;
+        if (Tally::kAlphaTextures || r->textured)
+            launch_gradient<Tally, true>(blocks, st, s, r->params, tile, sample_start, sample_count, gp, adjoint,
+                                         image, gradient);
+        else
+            launch_gradient<Tally, Tally::kAlphaTextures>(blocks, st, s, r->params, tile, sample_start, sample_count,
+                                                          gp, adjoint, image, gradient);
+    });
     WF_GRAD_CUDA(cudaGetLastError());
     WF_GRAD_CUDA(cudaStreamSynchronize(st));
     return WF_OK;

@@ -28,9 +28,9 @@ constexpr int kStackSize = 64;  // leaf depth <= kMaxBvhDepth (60) < 64
 // A tally type also fixes, at compile time, whether the traversal may meet
 // alpha-textured materials (kAlphaTextures) or primitives outside the BVHs
 // (kLinearLists: direct instances, static triangles, a direct list without a
-// BVH): the default types handle every scene; Opaque<T> compiles both out,
-// for kernels that the host launches only on scenes without either
-// (wf_scene::opaque).
+// BVH): the default types handle every scene, the wrappers below compile one
+// or both out, and with_variant picks the type for a scene
+// (wf_scene::opaque, wf_scene::listless).
 struct NoTally {
     static constexpr bool kCounts = false;
     static constexpr bool kAlphaTextures = true;
@@ -55,11 +55,24 @@ struct Opaque : Base {
     static constexpr bool kAlphaTextures = false;
     static constexpr bool kLinearLists = false;
 };
-// Alpha-textured materials, but every primitive in a BVH (wf_scene::listless).
+// No alpha-textured material, but primitives outside the BVHs.
+template <typename Base>
+struct Lists : Base {
+    static constexpr bool kAlphaTextures = false;
+};
+// Alpha-textured materials, but every primitive in a BVH.
 template <typename Base>
 struct Listless : Base {
     static constexpr bool kLinearLists = false;
 };
+// f with a value of the variant of Base for a scene.
+template <typename Base, typename F>
+auto with_variant(bool opaque, bool listless, F f) {
+    if (opaque && listless) return f(Opaque<Base>{});
+    if (opaque) return f(Lists<Base>{});
+    if (listless) return f(Listless<Base>{});
+    return f(Base{});
+}
 
 struct TraceState {
     float t;          // closestT
