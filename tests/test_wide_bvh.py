@@ -43,11 +43,12 @@ def check(tmp_path_factory):
             limits = np.random.default_rng(3).uniform(0.1, 20.0, len(rays))
         limits = np.ascontiguousarray(limits, np.float32)
         desc, keep = scene.desc()
-        counts = np.zeros(9, np.uint64)
+        counts = np.zeros(11, np.uint64)
         status = lib.wide_check(C.byref(desc), C.c_void_p(rays.ctypes.data), C.c_void_p(limits.ctypes.data),
                                 C.c_uint32(len(rays)), C.c_void_p(counts.ctypes.data))
         assert status == 0
-        names = ("closest", "any", "rays", "nodes", "wide_visits", "binary_visits", "usable", "redone", "hits")
+        names = ("closest", "any", "rays", "nodes", "wide_visits", "binary_visits", "usable", "redone", "hits", "tests",
+                 "binary_tests")
         got = dict(zip(names, (int(v) for v in counts)))
         assert got["closest"] == 0 and got["any"] == 0, got
         return got
@@ -295,6 +296,32 @@ def test_other_instance_transforms(check, kind, usable):
     o = rng.uniform(-9, 9, (60_000, 3))
     o[:, 1] = rng.uniform(0, 0.05, len(o))
     assert check(s, make_rays(o, unit(rng.normal(0, 1, o.shape))))["usable"] == usable
+
+
+def test_scenes_without_bvhs_and_past_the_range_are_traced_once(check):
+    """Linear lists alone, and rays or scenes for the BVH2s: no primitive is
+    tested twice."""
+    rng = np.random.default_rng(6)
+    rays = make_rays(rng.uniform(-2, 2, (2000, 3)).astype(np.float32), unit(rng.normal(0, 1, (2000, 3))))
+    s = Scene()
+    s.add_material(material(abi.MAT_DIFFUSE, (0.5, 0.5, 0.5)))
+    sp = np.zeros(9, abi.SPHERE_DTYPE)
+    sp["center"], sp["radius"], sp["accel"] = rng.uniform(-2, 2, (9, 3)), 0.4, abi.ACCEL_DIRECT
+    s.spheres = sp
+    w = soup(12, 3)
+    s.static_triangles = scenes.triangles(w[:, 0], w[:, 1], w[:, 2], 0)
+    got = check(s, rays)
+    assert got["redone"] == 0 and got["tests"] == got["binary_tests"] == 21 * len(rays)
+    mesh = mesh_scene(soup(300, 11))
+    mesh.spheres, mesh.static_triangles = sp, s.static_triangles
+    short = rays.copy()
+    short["direction"] *= np.float32(1e-8)
+    got = check(mesh, short)
+    assert got["redone"] == len(rays) and got["tests"] == got["binary_tests"]
+    huge = mesh_scene(soup(300, 11) * np.float32(1e9))
+    huge.spheres = sp
+    got = check(huge, rays)
+    assert got["usable"] == 0 and got["redone"] == len(rays) and got["tests"] == got["binary_tests"]
 
 
 def test_repository_scenes(check):

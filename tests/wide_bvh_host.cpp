@@ -95,19 +95,20 @@ void build_wide(Built& b) {
     v.wide.nodes = b.nodes.data();
     v.wide.triangles = b.triangles.data();
     v.wide.leaves = b.leaves.data();
-    v.wide.usable = usable && !trees.empty() ? 1u : 0u;
+    v.wide.usable = usable ? 1u : 0u;
 }
 }  // namespace
 
 // counts: [0] closest hits that differ, [1] occlusion answers that differ,
 // [2] rays, [3] wide nodes, [4] wide node visits, [5] BVH2 node visits,
-// [6] usable, [7] rays that the BVH2s decided, [8] hits
+// [6] usable, [7] rays that the BVH2s decided, [8] hits, [9] and [10]
+// primitive and instance tests of the wide and the BVH2 closest hits
 extern "C" int wide_check(const wf_scene_desc* desc, const wf_ray* rays, const float* limits, uint32_t count,
                           uint64_t* counts) {
     Built b;
     if (wf_status e = build_host_scene(desc, b.h)) return int(e);
     build_wide(b);
-    for (int k = 0; k < 9; ++k) counts[k] = 0;
+    for (int k = 0; k < 11; ++k) counts[k] = 0;
     counts[2] = count;
     counts[3] = b.nodes.size();
     counts[6] = b.v.wide.usable;
@@ -134,6 +135,8 @@ extern "C" int wide_check(const wf_scene_desc* desc, const wf_ray* rays, const f
         if (p != q) ++counts[1];
         counts[4] += wide.nodes;
         counts[5] += binary.nodes;
+        counts[9] += wide.triangles + wide.spheres + wide.instances;
+        counts[10] += binary.triangles + binary.spheres + binary.instances;
     }
     return 0;
 }

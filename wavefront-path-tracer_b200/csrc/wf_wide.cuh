@@ -88,17 +88,20 @@ WF_DEV float held_inverse(float d) {
     return copysignf(fminf(fabsf(1.0f / d), kInverseMax), d);
 }
 
-// Returns false for rays the wide test's bounds do not cover (NaN too: fmaxf
-// drops a NaN operand, the sum does not).
-WF_DEV bool wide_ray(WideRay& r, V3 o, V3 d) {
+// False for rays the wide test's bounds do not cover (NaN too: fmaxf drops a
+// NaN operand, the sum does not).
+WF_DEV bool ray_covered(V3 o, V3 d) {
+    float m = fmaxf(fabsf(d.x), fmaxf(fabsf(d.y), fabsf(d.z)));
+    float far = fmaxf(fabsf(o.x), fmaxf(fabsf(o.y), fabsf(o.z)));
+    return m >= 1.0e-6f && m <= 1.0e6f && far <= 1.0e7f && (o.x + o.y + o.z) + (d.x + d.y + d.z) < 1.0e9f;
+}
+
+WF_DEV void wide_ray(WideRay& r, V3 o, V3 d) {
     r.o = o;
     r.d = d;
     r.inv = V3{held_inverse(d.x), held_inverse(d.y), held_inverse(d.z)};
     uint32_t oct = (r.inv.x > 0.0f ? 1u : 0u) | (r.inv.y > 0.0f ? 2u : 0u) | (r.inv.z > 0.0f ? 4u : 0u);
     r.oct4 = oct * 0x01010101u;
-    float m = fmaxf(fabsf(d.x), fmaxf(fabsf(d.y), fabsf(d.z)));
-    float far = fmaxf(fabsf(o.x), fmaxf(fabsf(o.y), fabsf(o.z)));
-    return m >= 1.0e-6f && m <= 1.0e6f && far <= 1.0e7f && (o.x + o.y + o.z) + (d.x + d.y + d.z) < 1.0e9f;
 }
 
 // The BVH2's inverse direction: 1 / d itself (infinite for a zero component).
@@ -418,12 +421,19 @@ WF_DEV void lane_begin_direct(Lane& L, const DeviceScene& s) {
 }
 
 // Starts a ray: the linear stages of traceRay / isOccluded, then the TLAS
-// root.  t_max: a kAny ray's length.
+// root.  t_max: a kAny ray's length.  Rays and scenes that the wide test does
+// not cover go to the BVH2s before the linear stages, which those repeat.
 template <bool kAny, typename Tally, typename Sink>
 WF_DEV void lane_begin(Lane& L, const DeviceScene& s, Sink& sink, V3 o, V3 d, float t_max, Tally& tally) {
     L.state = kStageDone;
     L.t = t_max;
     L.size = 0;
+    L.world[0] = make_float4(o.x, o.y, o.z, 0.0f);
+    L.world[1] = make_float4(d.x, d.y, d.z, 0.0f);
+    if (!s.wide.usable || !ray_covered(o, d)) {
+        L.state |= kRedo;
+        return;
+    }
     if (kAny) {
         for (uint32_t i = 0; i < s.direct_sphere_count; ++i) {
             float t;
@@ -446,15 +456,11 @@ WF_DEV void lane_begin(Lane& L, const DeviceScene& s, Sink& sink, V3 o, V3 d, fl
         L.t = h.t;
         sink.hit(h.t, h.u, h.v, h.prim, h.inst);
     }
-    bool covered = wide_ray(L.r, o, d);
+    wide_ray(L.r, o, d);
     // (the TLAS's; lane_begin_direct has its own BVH's)
     if (!kAny) L.r.margin = cull_margin(o, s.tlas.box, s.wide.reach, s.wide.base);
-    lane_save_world(L);
-    if (!covered || !s.wide.usable) {
-        L.state |= kRedo;
-        return;
-    }
     if (s.tlas.root != kNoRoot) {
+        lane_save_world(L);
         float near_t;
         if (slab_box(o, exact_inverse(L.r), s.tlas.box, box_limit<kAny>(L), near_t)) {
             lane_stage(L, kStageTlas);
@@ -517,7 +523,8 @@ WF_DEV void lane_tlas_leaf(Lane& L, const DeviceScene& s, Sink& sink, uint32_t e
         L.state |= kRedo;
         return;
     }
-    bool covered = wide_ray(L.r, to_local_vector(in, L.r.o - instance_translation(in)), to_local_vector(in, L.r.d));
+    wide_ray(L.r, to_local_vector(in, L.r.o - instance_translation(in)), to_local_vector(in, L.r.d));
+    bool covered = ray_covered(L.r.o, L.r.d);
     if (!kAny) L.r.margin = cull_margin(L.r.o, f4xyz(root_lo), f4xyz(root_hi), kWideReach, 0.0f);
     float local_t;
     if (!covered || !exact_leaf_box(root_lo, root_hi, L.r, box_limit<kAny>(L), local_t) ||

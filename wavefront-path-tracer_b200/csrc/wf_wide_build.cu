@@ -54,10 +54,7 @@ __global__ void k_wide_emit(DeviceScene s, const BvhRef* roots, uint32_t count, 
 
 cudaError_t build_wide_bvh(DeviceScene& view, const std::vector<BvhRef>& roots, uint32_t node_count,
                            uint32_t tlas_root, std::vector<void*>& allocations, uint64_t& bytes) {
-    if (roots.empty()) {
-        view.wide.usable = 0u;
-        return cudaSuccess;
-    }
+    if (roots.empty()) return cudaSuccess;
     uint32_t root_count = uint32_t(roots.size());
     // Wide nodes other than the roots stand for distinct internal BVH2 nodes.
     size_t capacity = size_t(node_count) + root_count;
