@@ -103,6 +103,52 @@ def test_large_ray_batches_match_small_ones(cuda, which):
     dev.close()
 
 
+@pytest.mark.parametrize("lists", [False, True])
+@pytest.mark.parametrize("masked", [False, True])
+def test_ray_batches_do_not_depend_on_their_route(cuda, lists, masked):
+    """Which kernel traces a batch depends on the leaves of the scene's trees
+    (32 and 64 of them, 64 in the TLAS) and on its size.  Far and tiny spheres
+    that no ray meets change the count and must change nothing else."""
+    w, h = 64, 64
+    line = cuda.cuda.get_device_properties(0).multi_processor_count * 8 * 256
+    rng = np.random.default_rng(3)
+    rays = np.zeros(line + 33, abi.RAY_DTYPE)
+    rays["origin"] = rng.uniform(-0.9, 0.9, (len(rays), 3))
+    d = rng.normal(0, 1, (len(rays), 3))
+    rays["direction"] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    limit = rng.uniform(0.1, 3.0, len(rays)).astype(np.float32)
+    answers = []
+    for far in (0, 1, 32, 33, 33, 62, 63, 64):
+        scene = wfpt.Scene()
+        mat = scene.add_material(wfpt.material(abi.MAT_DIFFUSE, (0.5, 0.5, 0.5)))
+        half = scene.add_material(wfpt.material(abi.MAT_DIFFUSE, (0.5, 0.5, 0.5)))
+        if masked:
+            scene.materials[half]["alpha_masked"] = 1
+            scene.materials[half]["opacity"] = 0.0
+            scene.textures = [np.full((1, 1, 4), 255, np.uint8)]
+            scene.material_textures = scenes.material_textures()
+            scene.material_textures = np.concatenate(
+                [scene.material_textures, scenes.material_textures(albedo=scenes.texture_binding(0))])
+        v = (rng2 := np.random.default_rng(4)).uniform(-1, 1, (30, 1, 3)) + rng2.normal(0, 0.3, (30, 3, 3))
+        scene.add_mesh(scenes.triangles(*v.astype(np.float32).transpose(1, 0, 2), np.where(np.arange(30) % 3, mat, half)))
+        scene.instances = scenes.instance(0)
+        if lists:
+            scene.static_triangles = scenes.quad((-1, -0.7, 1), (1, -0.7, 1), (1, -0.7, -1), (-1, -0.7, -1), mat)
+        sp = np.zeros(far, abi.SPHERE_DTYPE)
+        sp["center"] = 1e6 + np.arange(far)[:, None]
+        sp["radius"], sp["material"], sp["accel"] = 1e-3, mat, abi.ACCEL_BVH
+        scene.spheres = sp
+        dev = wfpt.DeviceScene(scene)
+        for count in (1, 33, len(rays)):
+            answers.append((count, dev.trace_closest(rays[:count]).tobytes(),
+                            dev.trace_any(rays[:count], limit[:count]).tobytes()))
+        dev.close()
+    want = {count: (hits, occluded) for count, hits, occluded in answers[:3]}
+    assert 0 < sum(want[len(rays)][1]) < len(rays)
+    for count, hits, occluded in answers:
+        assert hits == want[count][0] and occluded == want[count][1]
+
+
 @pytest.mark.parametrize("capacity,pass_paths", [(0, 0), (33, 0), (300, 1021)])
 def test_batch_of_scenes_without_lights(cuda, capacity, pass_paths):
     """A batch of sphere fields shades without shadow rays; its images are

@@ -176,6 +176,11 @@ wf_status wf_scene_create(const wf_scene_desc* desc, wf_scene** out) {
     number(h.direct_bvh);
     number(h.tlas);
     uint32_t tlas_tree = h.tlas.wide;
+    s->tlas_leaves = uint32_t(h.tlas_leaves.size());
+    s->list_leaves = h.direct_bvh.root == kNoRoot ? 0u : h.direct_count;
+    s->tree_leaves = uint64_t(s->tlas_leaves) + s->list_leaves;
+    for (const Blas& b : h.blases)
+        if (b.bvh.root != kNoRoot) s->tree_leaves += b.count;
     v.wide = h.margins;
     up(&v.triangles, h.triangles);
     up(&v.normals, h.normals);

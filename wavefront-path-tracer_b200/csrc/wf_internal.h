@@ -112,4 +112,7 @@ struct wf_scene {
     wf::Box bounds{};
     int device = 0;
     int sm_count = 148;
+    uint32_t tlas_leaves = 0;    // instances and spheres of the TLAS
+    uint32_t list_leaves = 0;    // triangles of the direct list's BVH
+    uint64_t tree_leaves = 0;    // all of these and the meshes' triangles with a BVH
 };

@@ -991,28 +991,30 @@ WF_DEV void write_hit(const DeviceScene& s, V3 o, V3 d, const TraceState& h, wf_
 WF_DEV V3 ray_origin(const wf_ray& r) { return V3{r.origin[0], r.origin[1], r.origin[2]}; }
 WF_DEV V3 ray_direction(const wf_ray& r) { return V3{r.direction[0], r.direction[1], r.direction[2]}; }
 
-// A batch that the GPU holds at once: one ray per thread, bounded to 8 CTAs
-// of 128 per SM (64 registers).
-template <typename Tally>
+// One ray per thread, bounded to 8 CTAs of 128 per SM (64 registers); through
+// the BVH2s where kWide is false (ray_route).
+template <typename Tally, bool kWide>
 __global__ void __launch_bounds__(128, 8) k_trace_batch(const __grid_constant__ DeviceScene s, const wf_ray* rays,
                                                         uint32_t count, wf_hit* hits) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     V3 o = ray_origin(rays[i]), d = ray_direction(rays[i]);
     Tally tally;
-    write_hit(s, o, d, trace_closest(s, o, d, tally), &hits[i]);
+    write_hit(s, o, d, kWide ? trace_closest(s, o, d, tally) : trace_coherent(s, o, d, tally), &hits[i]);
 }
 
-template <typename Tally>
+template <typename Tally, bool kWide>
 __global__ void __launch_bounds__(128, 8) k_any_batch(const __grid_constant__ DeviceScene s, const wf_ray* rays,
                                                       const float* max_distance, uint32_t count, uint8_t* occluded) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     Tally tally;
-    occluded[i] = trace_any(s, ray_origin(rays[i]), ray_direction(rays[i]), max_distance[i], tally) ? 1 : 0;
+    V3 o = ray_origin(rays[i]), d = ray_direction(rays[i]);
+    occluded[i] = (kWide ? trace_any(s, o, d, max_distance[i], tally)
+                         : trace_any_binary(s, o, d, max_distance[i], tally)) ? 1 : 0;
 }
 
-// A larger batch: lane refill on one resident wave of CTAs.  Warp w of W
+// Lane refill on one resident wave of CTAs (ray_route).  Warp w of W
 // takes the blocks of 32 rays w, w + W, ... one after another and hands their
 // rays to its idle lanes, with no counter in memory (batches on several
 // streams would share it).  The records are completed, and the rays in doubt
@@ -2290,25 +2292,65 @@ wf_status renderer_profile(wf_renderer* r, wf_kernel_profile* out) {
 }
 
 namespace {
-// CTAs of 128 of the refilling batch kernels (8 per SM), and whether a batch
-// takes them: from twice the rays that they hold at once.
+// CTAs of 128 of the refilling batch kernels (8 per SM).
 uint32_t batch_ctas(const wf_scene* scene) { return uint32_t(scene->sm_count) * 8u; }
-bool large_batch(const wf_scene* scene, uint32_t count) { return count >= batch_ctas(scene) * 256u; }
+
+// How a batch of rays is traced.  The kernels are bound by the instructions
+// they issue (ncu: 59-71 % of the issue slots), so what decides is how much of
+// a ray's time is traversal.  2,000,001 random rays, microseconds, BVH2s /
+// wide BVH with one ray per thread / with refilled lanes:
+//                              closest hits        any hit
+//   Cornell box, 36 triangles   312  409  626    402  167  303
+//   24 triangles and a sphere   201  258  322    104  131  128
+//   walls in a list, one mesh   592  897  910    758  591  574
+//   two meshes, list beside     777 1095 2009   1075  724 1078
+//   dome of 112 triangles       666  545  881    424  304  475
+//   dome of 80,000              1154  858 1291    513  336  467
+//   484 spheres, 3 meshes       611  634  563    290  361  274
+//   120 meshes and spheres     1528 1333 1019   1112  507  423
+//   the same, a quad in a list 1653 1546 1262   1250  600  563
+//   direct list, 32,000         757  682  506    321  448  256
+//  * Trees of few leaves: the BVH2s.  A wide node decodes eight boxes and a
+//    closest hit is checked against its own box again, which a tree of five
+//    levels does not repay; an occlusion ray skips the second and needs half
+//    as many leaves.
+//  * Closest hits beside linear lists and few TLAS leaves: the BVH2s.
+//  * Many TLAS leaves, or a direct list's BVH: rays differ most in length
+//    there (misses, and instances entered in vain), so from twice the rays
+//    that the GPU holds at once on lanes are refilled; elsewhere that costs
+//    more than the idle lanes.
+// (Two copies of a scene in one place cost closest hits 2,757 -> 4,486 us
+// against the BVH2s alone: most rays tie and are traced by both.  Nothing
+// known before the launch tells such scenes.)
+enum class RayRoute { kBinary, kLanes, kBlocks };
+RayRoute ray_route(const wf_scene* scene, uint32_t count, bool any) {
+    bool many = scene->tlas_leaves >= 64 || scene->list_leaves >= 64;
+    if (!scene->view.wide.usable || scene->tree_leaves < (any ? 32u : 64u)) return RayRoute::kBinary;
+    if (!any && !many && !scene->listless()) return RayRoute::kBinary;
+    return many && count >= batch_ctas(scene) * 256u ? RayRoute::kBlocks : RayRoute::kLanes;
+}
 }  // namespace
 
 wf_status trace_closest_batch(const wf_scene* scene, const wf_ray* rays, uint32_t count, wf_hit* hits,
                               cudaStream_t stream) {
     if (count == 0) return WF_OK;
     uint32_t blocks = (count - 1) / 128 + 1;
-    if (large_batch(scene, count)) {
-        with_variant<NoTally>(scene->opaque(), scene->listless(), [&](auto tally) {
-            k_trace_blocks<decltype(tally)><<<batch_ctas(scene), 128, 0, stream>>>(scene->view, rays, count, hits);
-        });
-        k_finish_batch<<<blocks, 128, 0, stream>>>(scene->view, rays, count, hits);
+    RayRoute route = ray_route(scene, count, false);
+    if (route == RayRoute::kBinary) {
+        if (scene->opaque())
+            k_trace_batch<Opaque<NoTally>, false><<<blocks, 128, 0, stream>>>(scene->view, rays, count, hits);
+        else
+            k_trace_batch<NoTally, false><<<blocks, 128, 0, stream>>>(scene->view, rays, count, hits);
     } else {
         with_variant<NoTally>(scene->opaque(), scene->listless(), [&](auto tally) {
-            k_trace_batch<decltype(tally)><<<blocks, 128, 0, stream>>>(scene->view, rays, count, hits);
+            using Tally = decltype(tally);
+            if (route == RayRoute::kBlocks)
+                k_trace_blocks<Tally><<<batch_ctas(scene), 128, 0, stream>>>(scene->view, rays, count, hits);
+            else
+                k_trace_batch<Tally, true><<<blocks, 128, 0, stream>>>(scene->view, rays, count, hits);
         });
+        if (route == RayRoute::kBlocks)
+            k_finish_batch<<<blocks, 128, 0, stream>>>(scene->view, rays, count, hits);
     }
     WF_CUDA(cudaGetLastError());
     return WF_OK;
@@ -2318,16 +2360,25 @@ wf_status trace_any_batch(const wf_scene* scene, const wf_ray* rays, const float
                           uint8_t* occluded, cudaStream_t stream) {
     if (count == 0) return WF_OK;
     uint32_t blocks = (count - 1) / 128 + 1;
-    if (large_batch(scene, count)) {
-        with_variant<NoTally>(scene->opaque(), scene->listless(), [&](auto tally) {
-            k_any_blocks<decltype(tally)>
-                <<<batch_ctas(scene), 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
-        });
-        k_any_settle<<<blocks, 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
+    RayRoute route = ray_route(scene, count, true);
+    if (route == RayRoute::kBinary) {
+        if (scene->opaque())
+            k_any_batch<Opaque<NoTally>, false>
+                <<<blocks, 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
+        else
+            k_any_batch<NoTally, false><<<blocks, 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
     } else {
         with_variant<NoTally>(scene->opaque(), scene->listless(), [&](auto tally) {
-            k_any_batch<decltype(tally)><<<blocks, 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
+            using Tally = decltype(tally);
+            if (route == RayRoute::kBlocks)
+                k_any_blocks<Tally>
+                    <<<batch_ctas(scene), 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
+            else
+                k_any_batch<Tally, true>
+                    <<<blocks, 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
         });
+        if (route == RayRoute::kBlocks)
+            k_any_settle<<<blocks, 128, 0, stream>>>(scene->view, rays, max_distance, count, occluded);
     }
     WF_CUDA(cudaGetLastError());
     return WF_OK;
