@@ -11,7 +11,8 @@ meet:
   endless and no kernel is broken on purpose);
 * a queue that overflows: a shadow-ray queue smaller than one bounce needs;
 * a device allocation that fails: injected on the host (wf_test_fail_allocation)
-  at every allocation of scene and renderer creation in turn.
+  at every allocation of scene and renderer creation in turn (without memory
+  for the 8-wide BVH a scene keeps its BVH2s alone).
 
 After each failure the same renderer (or a new one) must render the oracle's
 framebuffer bit for bit."""
@@ -154,3 +155,47 @@ def test_injected_allocation_failures_free_everything(cuda):
     r.close()
     dev.close()
     assert same(got, expected_image(scene, cam, cfg, 3))
+
+
+def test_scene_without_memory_for_the_wide_bvh(cuda):
+    """Each of the wide BVH's four allocations fails in turn: the scene is
+    made, holds less memory and answers as before."""
+    lib = wfpt.library()
+    scene, cam = scenes.large_mesh(96, 54, terrain_quads=48, instance_count=12, instance_frequency=8, glass_spheres=4,
+                                   env_size=(64, 32))
+    rng = np.random.default_rng(1)
+    rays = np.zeros(5000, abi.RAY_DTYPE)
+    rays["origin"] = rng.uniform(-40, 40, (len(rays), 3)) + (0, 45, 0)
+    rays["direction"] = rng.normal(0, 1, (len(rays), 3))
+    limit = rng.uniform(1, 60, len(rays)).astype(np.float32)
+    cfg = wfpt.render_config(96, 54, max_depth=6)
+
+    def answers(dev):
+        r = wfpt.Renderer(dev, cam, cfg)
+        image = r.render_task((0, 0, 96, 54), 3, SPP)
+        r.close()
+        return image.tobytes(), dev.trace_closest(rays).tobytes(), dev.trace_any(rays, limit).tobytes()
+
+    dev = wfpt.DeviceScene(scene)
+    want = answers(dev)
+    whole = dev.info().device_bytes
+    dev.close()
+    made = failed = 0
+    try:
+        for k in range(10000):
+            lib.wf_test_fail_allocation(k)
+            try:
+                dev = wfpt.DeviceScene(scene)
+            except wfpt.WavefrontError:
+                failed += 1
+                continue
+            finally:
+                lib.wf_test_fail_allocation(-1)
+            made += 1
+            assert dev.info().device_bytes < whole and answers(dev) == want
+            dev.close()
+            if made == 4:
+                break
+    finally:
+        lib.wf_test_fail_allocation(-1)
+    assert failed >= 8

@@ -56,6 +56,8 @@ cudaError_t build_wide_bvh(DeviceScene& view, const std::vector<BvhRef>& roots, 
                            uint32_t tlas_root, std::vector<void*>& allocations, uint64_t& bytes) {
     if (roots.empty()) return cudaSuccess;
     uint32_t root_count = uint32_t(roots.size());
+    const size_t kept = allocations.size();
+    const uint64_t kept_bytes = bytes;
     // Wide nodes other than the roots stand for distinct internal BVH2 nodes.
     size_t capacity = size_t(node_count) + root_count;
     // one allocation: counters, bases, items, root refs (each part's alignment
@@ -108,7 +110,16 @@ cudaError_t build_wide_bvh(DeviceScene& view, const std::vector<BvhRef>& roots, 
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     cudaFree(scratch);
-    if (e == cudaSuccess) {
+    if (e != cudaSuccess) {
+        for (size_t i = kept; i < allocations.size(); ++i) cudaFree(allocations[i]);
+        allocations.resize(kept);
+        bytes = kept_bytes;
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            view.wide.usable = 0u;
+            return cudaSuccess;
+        }
+    } else {
         view.wide.nodes = nodes;
         view.wide.triangles = triangles;
         view.wide.leaves = leaves;
