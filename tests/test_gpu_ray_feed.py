@@ -172,3 +172,24 @@ def test_batch_of_scenes_without_lights(cuda, capacity, pass_paths):
     batch.close()
     for job in jobs:
         job["scene"].close()
+
+
+@pytest.mark.parametrize("which,direct", [("spheres", True), ("cornell", False)])
+def test_stage_profile_times_the_kernels_of_the_graph(cuda, which, direct):
+    """A scene that shades without shadow rays has no shadow and finalize
+    launches; the profiled passes add the same samples as the graph."""
+    w, h, depth = 65, 33, 6
+    scene, cam = _scene(which, w, h)
+    dev = wfpt.DeviceScene(scene)
+    cfg = wfpt.render_config(w, h, max_depth=depth, rr_start_depth=4)
+    r = wfpt.Renderer(dev, cam, cfg)
+    p = r.profile_sample()
+    assert p["shade"]["launches"] == p["trace"]["launches"] == depth
+    assert p["shadow"]["launches"] == p["finalize"]["launches"] == (0 if direct else depth)
+    assert p["shadow_rays"] == 0 if direct else p["shadow_rays"] > 0
+    plain = wfpt.Renderer(dev, cam, cfg)  # the timed pass and the counting one are samples 0 and 1
+    want = plain.render_task((0, 0, w, h), 0, 2)
+    assert np.array_equal(r.download().view(np.uint32), want.view(np.uint32))
+    r.close()
+    plain.close()
+    dev.close()

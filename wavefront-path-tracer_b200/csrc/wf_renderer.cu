@@ -2151,6 +2151,8 @@ wf_status renderer_profile(wf_renderer* r, wf_kernel_profile* out) {
         if (!r->tally) WF_CUDA(alloc(r, &r->tally, 2));
         const DeviceScene& s = r->scene->view;
         uint32_t cap = r->capacity;
+        // as the graph, unless an environment came after it
+        const bool direct = r->direct && r->scene->eventless();
         for (int pass = 0; pass < 2; ++pass) {
             bool count = pass == 1;
             if (count) WF_CUDA(cudaMemsetAsync(r->tally, 0, 2 * sizeof(TallyTotals), st));
@@ -2191,6 +2193,13 @@ wf_status renderer_profile(wf_renderer* r, wf_kernel_profile* out) {
                             k_scatter<<<grid(r, 3, cap, 256), 256, 0, st>>>(cur_count, r->shade_key,
                                                                              r->shade_order, r->counters);
                         }
+                        if (direct) {
+                            launch_shade_direct(r, grid(r, 1, cap, r->block_shade), r->block_shade, st, s, r->params,
+                                                r->paths, r->queue[cur], cur_count, r->hit_a, r->hit_inst,
+                                                r->counters, r->queue[nxt], next_count, cap,
+                                                r->sort_shading ? r->shade_order : nullptr, r->framebuffer, r->tile);
+                            return;
+                        }
                         launch_shade(r, grid(r, 1, cap, r->block_shade), r->block_shade, st, 
                             s, r->params, r->paths, r->queue[cur], cur_count, r->hit_a, r->hit_inst, r->terms,
                             r->shade_out, r->shadow_origin, r->shadow_dir, r->shadow_capacity, r->counters,
@@ -2222,6 +2231,7 @@ wf_status renderer_profile(wf_renderer* r, wf_kernel_profile* out) {
                         WF_CUDA(cudaGetLastError());
                         shade();
                         WF_CUDA(cudaGetLastError());
+                        if (direct) continue;
                         if (gathers) gather();
                         shadow();
                         WF_CUDA(cudaGetLastError());
@@ -2235,6 +2245,7 @@ wf_status renderer_profile(wf_renderer* r, wf_kernel_profile* out) {
                         for (int step = 0; step < 5; ++step) {
                             int k = order[step];
                             if (k == 4 && !gathers) continue;
+                            if (direct && k > 1) continue;  // k_shade_direct ends the bounce
                             wf_status e = k == 0   ? timed(kinds[k], trace)
                                           : k == 1 ? timed(kinds[k], shade)
                                           : k == 2 ? timed(kinds[k], shadow)
@@ -2242,11 +2253,13 @@ wf_status renderer_profile(wf_renderer* r, wf_kernel_profile* out) {
                                                    : timed(kinds[k], gather);
                             if (e) return e;
                             out->bounce_milliseconds[k][pb] += last_ms;
-                            if (k == 2) {  // after the shadow kernel: rays traced and shadow rays of this bounce
-                                uint32_t rays[2];
+                            if (k == (direct ? 1 : 2)) {  // rays traced and shadow rays of this bounce
+                                uint32_t rays[2] = {0, 0};
                                 if (wf_status e2 = read_back(&rays[0], cur_count, sizeof(uint32_t))) return e2;
-                                if (wf_status e2 = read_back(&rays[1], &r->counters->shadow_count, sizeof(uint32_t)))
-                                    return e2;
+                                if (!direct)
+                                    if (wf_status e2 = read_back(&rays[1], &r->counters->shadow_count,
+                                                                 sizeof(uint32_t)))
+                                        return e2;
                                 out->bounce_extension_rays[pb] += rays[0];
                                 out->bounce_shadow_rays[pb] += std::min(rays[1], r->shadow_capacity);
                             }
