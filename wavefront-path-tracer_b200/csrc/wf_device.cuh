@@ -10,8 +10,9 @@
 //     (lxy | rxy | lrz | children), so one node visit is four 16-byte loads and
 //     tests two boxes.  Child refs >= 0 are node indices, < 0 are ~leaf.
 //   * wide nodes: the same trees collapsed to 8 children per 80-byte node with
-//     8-bit box planes; every traversal uses them, and the BVH2 nodes decide
-//     the rays whose result could depend on the visit order (wf_wide.cuh).
+//     8-bit box planes; every traversal but camera rays, frame guides and the
+//     ray batches of shallow scenes uses them, and the BVH2 nodes decide the
+//     rays whose result could depend on the visit order (wf_wide.cuh).
 //   * spheres: float4 (center, radius) + material.
 // The arithmetic helpers reproduce the reference's Vec3 operators
 // (include/core/vec3.cuh:6-99) operation for operation so that, compiled with
@@ -144,7 +145,7 @@ struct alignas(16) WideLeaf {
     float4 lo;         // leaf box lo, .w = tlas_leaves word ((is_sphere << 31) | index)
     float4 hi;         // leaf box hi, .w = wide root of the BLAS (kNoWide: none)
     float4 root_lo;    // BLAS root box lo, .w = material override
-    float4 root_hi;    // BLAS root box hi, .w = BLAS index
+    float4 root_hi;    // BLAS root box hi
 };
 static_assert(sizeof(WideLeaf) == 112, "TLAS leaf record");
 

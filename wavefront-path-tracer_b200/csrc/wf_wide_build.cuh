@@ -242,8 +242,7 @@ WF_HDI WideNode wide_record(const DeviceScene& s, const Collapsed& c, bool tlas,
                     leaf.hi.w = bits_to_float(b.bvh.root == kNoRoot ? kNoWide : b.bvh.wide);
                     leaf.root_lo = make_float4(b.bvh.box.lo[0], b.bvh.box.lo[1], b.bvh.box.lo[2],
                                                bits_to_float(in.material_override));
-                    leaf.root_hi = make_float4(b.bvh.box.hi[0], b.bvh.box.hi[1], b.bvh.box.hi[2],
-                                               bits_to_float(in.blas));
+                    leaf.root_hi = make_float4(b.bvh.box.hi[0], b.bvh.box.hi[1], b.bvh.box.hi[2], 0.0f);
                 }
                 leaves[n.leaf_base + entry] = leaf;
             } else {
