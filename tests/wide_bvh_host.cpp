@@ -35,29 +35,20 @@ void build_wide(Built& b) {
     for (Blas& x : b.h.blases) number(x.bvh);
     number(b.h.direct_bvh);
     number(b.h.tlas);
-    std::vector<uint32_t> items;
-    for (uint32_t i = 0; i < trees.size(); ++i) {
-        uint32_t item = trees[i].root < 0 ? (kLeafItem | uint32_t(~trees[i].root)) : uint32_t(trees[i].root);
-        items.push_back(item | (i == b.h.tlas.wide ? kTlasItem : 0u));
-    }
+    // as build_wide_bvh: one node at a time, with room for every BVH2 node
+    uint32_t counters[3] = {uint32_t(trees.size()), 0, 0};
+    std::vector<uint32_t> items(b.h.nodes.size() + trees.size());
+    for (uint32_t i = 0; i < trees.size(); ++i) items[i] = root_item(trees[i], i == b.h.tlas.wide);
     bool usable = b.h.margins.usable != 0;
     std::vector<uint2> bases;
-    uint32_t triangle_count = 0, leaf_count = 0;
-    for (uint32_t i = 0; i < items.size(); ++i) {
-        Collapsed c;
-        collapse(b.h.nodes.data(), items[i], trees.data() + i, c);
-        bool tlas = (items[i] & kTlasItem) != 0;
-        uint32_t& entries = tlas ? leaf_count : triangle_count;
-        bases.push_back(make_uint2(uint32_t(items.size()), entries));
-        entries += uint32_t(c.leaves);
-        for (int k = 0; k < kWide; ++k) {
-            if (c.count[k] == 0) continue;
-            for (int a = 0; a < 3; ++a)
-                usable = usable && std::fabs(c.child[k].lo[a]) <= kWideMaxCoordinate &&
-                         std::fabs(c.child[k].hi[a]) <= kWideMaxCoordinate;
-            if (c.count[k] < 0) items.push_back(uint32_t(c.child[k].ref) | (tlas ? kTlasItem : 0u));
-        }
+    for (uint32_t i = 0; i < counters[0]; ++i) {
+        bool fits;
+        bases.push_back(number_children(
+            b.h.nodes.data(), items[i], trees.data() + i, items.data(),
+            [&](int k, uint32_t n) { uint32_t old = counters[k]; counters[k] += n; return old; }, fits));
+        usable = usable && fits;
     }
+    items.resize(counters[0]);
     DeviceScene& v = b.v;
     v.triangles = b.h.triangles.data();
     v.nodes = b.h.nodes.data();
@@ -84,8 +75,8 @@ void build_wide(Built& b) {
     v.direct_instance_count = uint32_t(b.h.direct_instances.size());
     v.any_alpha_reject = b.h.any_alpha_reject ? 1u : 0u;
     v.wide = b.h.margins;
-    b.triangles.resize(triangle_count);
-    b.leaves.resize(leaf_count);
+    b.triangles.resize(counters[1]);
+    b.leaves.resize(counters[2]);
     for (uint32_t i = 0; i < items.size(); ++i) {
         Collapsed c;
         collapse(v.nodes, items[i], trees.data() + i, c);

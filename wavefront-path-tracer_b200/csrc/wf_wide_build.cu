@@ -23,21 +23,9 @@ __global__ void k_wide_number(const BvhNode* nodes, const BvhRef* roots, uint32_
                               uint32_t* items, uint2* bases, uint32_t* counters) {
     uint32_t i = begin + blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= end) return;
-    uint32_t item = items[i];
-    bool tlas = (item & kTlasItem) != 0;
-    Collapsed c;
-    collapse(nodes, item, roots + i, c);
-    uint32_t base = c.internal ? atomicAdd(&counters[0], uint32_t(c.internal)) : 0u;
-    uint32_t leaf_base = c.leaves ? atomicAdd(&counters[tlas ? 2 : 1], uint32_t(c.leaves)) : 0u;
-    bases[i] = make_uint2(base, leaf_base);
-    bool fits = true;
-    for (int slot = 0; slot < kWide; ++slot) {
-        if (c.count[slot] == 0) continue;
-        for (int a = 0; a < 3; ++a)
-            fits = fits && fabsf(c.child[slot].lo[a]) <= kWideMaxCoordinate &&
-                   fabsf(c.child[slot].hi[a]) <= kWideMaxCoordinate;
-        if (c.count[slot] < 0) items[base++] = uint32_t(c.child[slot].ref) | (tlas ? kTlasItem : 0u);
-    }
+    bool fits;
+    bases[i] = number_children(
+        nodes, items[i], roots + i, items, [&](int k, uint32_t n) { return atomicAdd(&counters[k], n); }, fits);
     if (!fits) counters[3] = 1u;
 }
 
@@ -73,10 +61,7 @@ cudaError_t build_wide_bvh(DeviceScene& view, const std::vector<BvhRef>& roots, 
     uint32_t host[4] = {root_count, 0, 0, 0};
     if (e == cudaSuccess) {
         std::vector<uint32_t> first(root_count);
-        for (uint32_t i = 0; i < root_count; ++i) {
-            first[i] = roots[i].root < 0 ? (kLeafItem | uint32_t(~roots[i].root)) : uint32_t(roots[i].root);
-            if (i == tlas_root) first[i] |= kTlasItem;
-        }
+        for (uint32_t i = 0; i < root_count; ++i) first[i] = root_item(roots[i], i == tlas_root);
         e = cudaMemcpy(items, first.data(), root_count * sizeof(uint32_t), cudaMemcpyHostToDevice);
     }
     if (e == cudaSuccess) e = cudaMemcpy(counters, host, sizeof(host), cudaMemcpyHostToDevice);

@@ -146,6 +146,36 @@ WF_HDI void collapse(const BvhNode* nodes, uint32_t item, const BvhRef* root, Co
     }
 }
 
+// Numbers the children of the wide node that `item` stands for: the first
+// entries of its internal children (appended to `items`) and of its leaves.
+// add(k, n) adds n to counter k and returns what it held: [0] nodes, [1]
+// triangles, [2] TLAS leaves.  `fits`: whether its boxes are in the range of
+// the ray test.
+template <typename Add>
+WF_HDI uint2 number_children(const BvhNode* nodes, uint32_t item, const BvhRef* root, uint32_t* items, Add add,
+                             bool& fits) {
+    bool tlas = (item & kTlasItem) != 0;
+    Collapsed c;
+    collapse(nodes, item, root, c);
+    uint32_t base = c.internal ? add(0, uint32_t(c.internal)) : 0u;
+    uint32_t leaf_base = c.leaves ? add(tlas ? 2 : 1, uint32_t(c.leaves)) : 0u;
+    fits = true;
+    uint32_t next = base;
+    for (int slot = 0; slot < kWide; ++slot) {
+        if (c.count[slot] == 0) continue;
+        for (int a = 0; a < 3; ++a)
+            fits = fits && fabsf(c.child[slot].lo[a]) <= kWideMaxCoordinate &&
+                   fabsf(c.child[slot].hi[a]) <= kWideMaxCoordinate;
+        if (c.count[slot] < 0) items[next++] = uint32_t(c.child[slot].ref) | (tlas ? kTlasItem : 0u);
+    }
+    return make_uint2(base, leaf_base);
+}
+
+// The first items: the roots of the trees.
+WF_HDI uint32_t root_item(const BvhRef& tree, bool tlas) {
+    return (tree.root < 0 ? (kLeafItem | uint32_t(~tree.root)) : uint32_t(tree.root)) | (tlas ? kTlasItem : 0u);
+}
+
 // Grid of one axis: cells of 2^e with 252 of them at least as long as the
 // node, no finer than the rounding of its coordinates, 2^-20 of its longest
 // side or 4e-12 (the ray test's bounds, wf_wide.cuh); the origin lies one
