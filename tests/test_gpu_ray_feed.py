@@ -193,3 +193,21 @@ def test_stage_profile_times_the_kernels_of_the_graph(cuda, which, direct):
     r.close()
     plain.close()
     dev.close()
+
+
+def test_scene_creation_does_not_wait_for_other_streams(cuda):
+    """A scene is made while another stream is busy for about a second."""
+    torch = cuda
+    scene, _ = _scene("cornell", 64, 64)
+    wfpt.DeviceScene(scene).close()  # loads the kernels
+    torch.cuda.synchronize()
+    busy = torch.cuda.Stream()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(2_000_000_000)
+        end = torch.cuda.Event()
+        end.record()
+    dev = wfpt.DeviceScene(scene)
+    still_busy = not end.query()
+    torch.cuda.synchronize()
+    dev.close()
+    assert still_busy

@@ -25,18 +25,23 @@ namespace {
 std::atomic<long long> g_fail_allocation{-1};
 }  // namespace
 
-cudaError_t device_alloc(void** p, size_t bytes) {
+// Whether this allocation is the one to fail.
+static bool fail_this_allocation() {
     long long left = g_fail_allocation.load();
-    while (left >= 0) {
-        if (g_fail_allocation.compare_exchange_weak(left, left - 1)) {
-            if (left == 0) {
-                *p = nullptr;
-                return cudaErrorMemoryAllocation;
-            }
-            break;
-        }
-    }
-    return cudaMalloc(p, bytes);
+    while (left >= 0)
+        if (g_fail_allocation.compare_exchange_weak(left, left - 1)) return left == 0;
+    return false;
+}
+
+cudaError_t device_alloc(void** p, size_t bytes) {
+    if (!fail_this_allocation()) return cudaMalloc(p, bytes);
+    *p = nullptr;
+    return cudaErrorMemoryAllocation;
+}
+cudaError_t device_alloc_async(void** p, size_t bytes, cudaStream_t stream) {
+    if (!fail_this_allocation()) return cudaMallocAsync(p, bytes, stream);
+    *p = nullptr;
+    return cudaErrorMemoryAllocation;
 }
 }  // namespace wf
 

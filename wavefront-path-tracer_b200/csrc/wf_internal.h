@@ -19,6 +19,9 @@ wf_status fail(wf_status status, const char* format, ...);
 // test can make one of them fail (wf_test_fail_allocation) and check that
 // the entry point frees what it allocated and reports WF_ERR_OOM.
 cudaError_t device_alloc(void** p, size_t bytes);
+// ... or, for scratch memory that is given back with cudaFreeAsync (cudaFree
+// waits for every stream of the device), through this one.
+cudaError_t device_alloc_async(void** p, size_t bytes, cudaStream_t stream);
 
 // The scene after the host build, in device layout (see wf_device.cuh).
 struct HostScene {

@@ -52,8 +52,9 @@ cudaError_t build_wide_bvh(DeviceScene& view, const std::vector<BvhRef>& roots, 
     // divides the size of those before it)
     static_assert(sizeof(BvhRef) % sizeof(uint32_t) == 0 && alignof(BvhRef) == sizeof(uint32_t), "packed after words");
     char* scratch = nullptr;
-    cudaError_t e = device_alloc(reinterpret_cast<void**>(&scratch),
-                                 16 + capacity * (sizeof(uint2) + sizeof(uint32_t)) + root_count * sizeof(BvhRef));
+    cudaError_t e = device_alloc_async(
+        reinterpret_cast<void**>(&scratch),
+        16 + capacity * (sizeof(uint2) + sizeof(uint32_t)) + root_count * sizeof(BvhRef), cudaStreamLegacy);
     uint32_t* counters = reinterpret_cast<uint32_t*>(scratch);
     uint2* bases = reinterpret_cast<uint2*>(scratch + 16);
     uint32_t* items = reinterpret_cast<uint32_t*>(bases + capacity);
@@ -93,8 +94,10 @@ cudaError_t build_wide_bvh(DeviceScene& view, const std::vector<BvhRef>& roots, 
         k_wide_emit<<<(host[0] + 127) / 128, 128>>>(view, root_refs, host[0], items, bases, nodes, triangles, leaves);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    cudaFree(scratch);
+    // the legacy stream alone: renders on other streams go on
+    if (scratch) cudaFreeAsync(scratch, cudaStreamLegacy);
+    cudaError_t waited = cudaStreamSynchronize(cudaStreamLegacy);
+    if (e == cudaSuccess) e = waited;
     if (e != cudaSuccess) {
         for (size_t i = kept; i < allocations.size(); ++i) cudaFree(allocations[i]);
         allocations.resize(kept);
