@@ -19,7 +19,6 @@ static inline float __fmaf_rn(float a, float b, float c) { return std::fma(a, b,
 static inline int __popc(unsigned v) { return __builtin_popcount(v); }
 static inline int __ffs(int v) { return __builtin_ffs(v); }
 static inline int __clz(int v) { return v ? __builtin_clz(unsigned(v)) : 32; }
-static inline unsigned __activemask() { return 1u; }
 static inline bool __any_sync(unsigned, bool p) { return p; }
 static inline uint32_t __byte_perm(uint32_t x, uint32_t y, uint32_t s) {
     uint64_t both = uint64_t(y) << 32 | x;

@@ -618,15 +618,12 @@ WF_DEV void lane_finish(Lane& L, const DeviceScene& s, Sink& sink, Tally& tally)
 WF_DEV bool lane_doubt(const Lane& L) { return (L.state & (kTie | kRedo)) && !(L.state & kHit); }
 
 // ------------------------------------------------- one ray to its end
-// The loop keeps the warp's lanes together: without the vote, lanes that
-// leave a step by different branches drift apart and run one by one (frame
-// guides 2.4 -> 6.4 ms).
+// (Without a warp vote: keeping the lanes together by one at every step costs
+// the inverse step 3 %, 9.00 against 8.70 ms, and small ray batches 2-4 %.)
 template <bool kAny, typename Tally, typename Sink>
 WF_DEV bool lane_run(Lane& L, const DeviceScene& s, Sink& sink, V3 o, V3 d, float t_max, Tally& tally) {
-    unsigned warp = __activemask();
     lane_begin<kAny>(L, s, sink, o, d, t_max, tally);
-    while (__any_sync(warp, !lane_done(L)))
-        if (!lane_done(L)) lane_step<kAny>(L, s, sink, tally);
+    while (!lane_done(L)) lane_step<kAny>(L, s, sink, tally);
     lane_finish<kAny>(L, s, sink, tally);
     if (!lane_doubt(L)) return (L.state & kHit) != 0;
     V3 wo = f4xyz(L.world[0]), wd = f4xyz(L.world[1]);
