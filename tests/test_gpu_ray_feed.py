@@ -211,3 +211,19 @@ def test_scene_creation_does_not_wait_for_other_streams(cuda):
     torch.cuda.synchronize()
     dev.close()
     assert still_busy
+
+
+def test_guides_do_not_depend_on_the_tile(cuda):
+    """Pixels go to the warps in blocks for tiles of two resident waves (16
+    CTAs of 128 an SM) and more, in rows for smaller ones."""
+    line = cuda.cuda.get_device_properties(0).multi_processor_count * 16 * 128
+    w, h = 701, line // 701 + 3
+    scene, cam = _scene("mesh", w, h)
+    dev = wfpt.DeviceScene(scene)
+    whole = dev.frame_guides(cam, w, h)
+    assert w * h > line and 0 < int((whole["valid"] != 0).sum()) < w * h
+    for x, y, tw, th in ((0, 0, w, h // 2), (0, h // 2, 333, h - h // 2), (333, h // 2, w - 333, h - h // 2),
+                         (0, 0, w, h - 4), (17, 5, 1, 1), (3, 7, 31, 5)):
+        tile = dev.frame_guides(cam, w, h, tile=(x, y, tw, th))
+        assert tile.tobytes() == np.ascontiguousarray(whole[y:y + th, x:x + tw]).tobytes()
+    dev.close()

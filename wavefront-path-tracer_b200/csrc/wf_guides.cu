@@ -59,13 +59,21 @@ WF_DEV bool closest_surface(const DeviceScene& s, V3 o, V3 d, SurfaceHit& sh) {
 // registers, 6 CTAs) and 3.78 ms at 72 registers, all with a warp's pixels in
 // a row; in blocks of 8 x 4 the bounded kernel went from 2.92 to 2.32 ms at
 // the frame it is timed on (700 k triangles, download included).
+//
+// kBlocks: a warp's pixels form a block of 8 x 4, else a run of a row.  Blocks
+// visit fewer nodes, but the slow pixels of a frame then meet in one warp,
+// which a frame of little more than one resident wave waits for.  Rows /
+// blocks in us, scenes of 8 k, 51 k and 320 k terrain triangles: 160x90
+// 308/398, 437/384, 509/492; 640x360 346/389, 538/480, 706/721; 960x540
+// 450/435, 687/597, 992/897; 1280x720 683/568, 972/794, 1396/1212.
+template <bool kBlocks>
 __global__ void __launch_bounds__(128, 8) k_frame_guides(const __grid_constant__ DeviceScene s, Camera camera,
                                                       Camera previous, uint32_t has_previous, uint32_t width,
                                                       uint32_t height, uint32_t x0, uint32_t y0, uint32_t tile_w,
                                                       uint32_t tile_h, wf_frame_guide* out) {
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= tile_w * tile_h) return;
-    uint2 at = tile_pixel(k, tile_w, tile_h);
+    uint2 at = kBlocks ? tile_pixel(k, tile_w, tile_h) : make_uint2(k % tile_w, k / tile_w);
     uint32_t x = x0 + at.x, y = y0 + at.y, index = at.y * tile_w + at.x;
     V3 o, d;
     camera_ray(camera, (x + 0.5f) / width, (y + 0.5f) / height, o, d);
@@ -133,8 +141,10 @@ wf_status frame_guides(const wf_scene* scene, const wf_camera* camera, const wf_
     Camera now = device_camera(*camera);
     Camera before = previous ? device_camera(*previous) : now;
     uint32_t blocks = uint32_t((count + 127) / 128);
-    k_frame_guides<<<blocks, 128, 0, stream>>>(scene->view, now, before, previous ? 1u : 0u, width, height, x, y, w, h,
-                                              guides);
+    // blocks of pixels from two resident waves on
+    auto kernel = blocks >= uint32_t(scene->sm_count) * 16u ? k_frame_guides<true> : k_frame_guides<false>;
+    kernel<<<blocks, 128, 0, stream>>>(scene->view, now, before, previous ? 1u : 0u, width, height, x, y, w, h,
+                                       guides);
     WF_CUDA(cudaGetLastError());
     return WF_OK;
 }
