@@ -152,6 +152,22 @@ def test_direction_lengths_and_far_origins(check, length):
     check(mesh_scene(v), far)
 
 
+@pytest.mark.parametrize("scale,usable", [(1e7, 1), (4e8, 1), (6e8, 1), (2e9, 0)])
+def test_large_coordinates(check, scale, usable):
+    """Coordinates up to 1e9 (the soup's reach 1.6 times the scale), rays with
+    zero and denormal components among them, from within and from far away,
+    with short and long directions."""
+    v = soup(800, 4, flat=True) / np.float32(1.7)
+    s = mesh_scene((v * np.float32(scale)).astype(np.float32),
+                   scenes.instance(0), scenes.instance(0, (0.1 * scale, 0, 0), 0.5, 30.0))
+    for length in (1.0, 1e-4, 1e4):
+        rays = hard_rays(v.reshape(-1, 3), 1.0, 6)
+        rays["origin"] *= np.float32(0.6 * scale)
+        rays["direction"] *= np.float32(length)
+        got = check(s, rays, np.random.default_rng(1).uniform(0, 3 * scale / length, len(rays)))
+        assert got["usable"] == usable and (got["hits"] > 0) and (not usable or got["redone"] < len(rays) // 2)
+
+
 def test_boxes_past_the_range_and_odd_rays(check):
     v = soup(300, 11)
     assert check(mesh_scene(v * np.float32(1e9)), hard_rays(v.reshape(-1, 3) * 1e9, 1e9, 1))["usable"] == 0

@@ -151,7 +151,7 @@ static_assert(sizeof(WideLeaf) == 112, "TLAS leaf record");
 
 // The wide traversal's error bounds hold for coordinates up to this size
 // (wf_wide.cuh); larger scenes use the BVH2s alone.
-constexpr float kWideMaxCoordinate = 1.0e7f;
+constexpr float kWideMaxCoordinate = 1.0e9f;
 
 // Least values of WideBvh's margins, and the largest reach with which culling
 // is still worth its nodes (a matrix and its inverse 1/2048 apart).

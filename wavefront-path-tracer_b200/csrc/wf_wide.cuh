@@ -57,11 +57,11 @@
 // into the second byte of 1.0f.  Rounding moves it by less than
 // 2^-8 cells + 2^-21 of the distance against the BVH2's own slab value; the
 // builder leaves 1/64 cell on either side and the test 2^-15 of the distance
-// (kSlack).  1 / d is held to 2^90: the spare of the smallest cell (4e-12)
-// times that still reaches past any distance a direction of at least 1e-6
-// covers (3.5e13).  The bounds on origin (1e7), direction (1e-6 to 1e6) and
-// scene coordinates (kWideMaxCoordinate) keep every product finite.  Rays
-// outside them take the BVH2s.
+// (kSlack).  1 / d is held to 2^88: the spare of the smallest cell (1e-9)
+// times that (4.8e15) still reaches past any distance a direction of at least
+// 1e-6 covers (3.5e15).  The bounds on origin (1e9), direction (1e-6 to 1e6)
+// and scene coordinates (kWideMaxCoordinate) keep every product finite: cells
+// are at most 2^23, S at most 2^126.  Rays outside them take the BVH2s.
 #pragma once
 
 #include "wf_traverse.cuh"
@@ -82,7 +82,7 @@ struct WideRay {
     uint32_t oct4;  // per byte: bit a set when inv's component a is positive
     float margin;   // how far outside its box a primitive's distance may lie
 };
-constexpr float kInverseMax = 1.2379400392853803e27f;  // 2^90
+constexpr float kInverseMax = 3.0948500982134507e26f;  // 2^88
 
 WF_DEV float held_inverse(float d) {
     return copysignf(fminf(fabsf(1.0f / d), kInverseMax), d);
@@ -93,7 +93,7 @@ WF_DEV float held_inverse(float d) {
 WF_DEV bool ray_covered(V3 o, V3 d) {
     float m = fmaxf(fabsf(d.x), fmaxf(fabsf(d.y), fabsf(d.z)));
     float far = fmaxf(fabsf(o.x), fmaxf(fabsf(o.y), fabsf(o.z)));
-    return m >= 1.0e-6f && m <= 1.0e6f && far <= 1.0e7f && (o.x + o.y + o.z) + (d.x + d.y + d.z) < 1.0e9f;
+    return m >= 1.0e-6f && m <= 1.0e6f && far <= kWideMaxCoordinate && (o.x + o.y + o.z) + (d.x + d.y + d.z) < 1.0e11f;
 }
 
 WF_DEV void wide_ray(WideRay& r, V3 o, V3 d) {

@@ -178,11 +178,11 @@ WF_HDI uint32_t root_item(const BvhRef& tree, bool tlas) {
 
 // Grid of one axis: cells of 2^e with 252 of them at least as long as the
 // node, no finer than the rounding of its coordinates, 2^-20 of its longest
-// side or 4e-12 (the ray test's bounds, wf_wide.cuh); the origin lies one
+// side or 1e-9 (the ray test's bounds, wf_wide.cuh); the origin lies one
 // cell below the node.
 WF_HDI void axis_grid(float lo, float hi, float longest, float& origin, int& exponent) {
     float cell = fmaxf((hi - lo) * (1.0f / 252.0f), fmaxf(fabsf(lo), fabsf(hi)) * 2.384185791015625e-7f);
-    cell = fmaxf(cell, fmaxf(longest * 9.5367431640625e-7f, 4.0e-12f));
+    cell = fmaxf(cell, fmaxf(longest * 9.5367431640625e-7f, 1.0e-9f));
     int e;
     float m = frexpf(cell, &e);  // cell = m 2^e, m in [0.5, 1)
     if (m == 0.5f) --e;
