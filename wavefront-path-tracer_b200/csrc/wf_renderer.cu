@@ -1011,7 +1011,7 @@ __global__ void __launch_bounds__(128, 8) k_any_batch(const __grid_constant__ De
     Tally tally;
     V3 o = ray_origin(rays[i]), d = ray_direction(rays[i]);
     occluded[i] = (kWide ? trace_any(s, o, d, max_distance[i], tally)
-                         : trace_any_binary(s, o, d, max_distance[i], tally)) ? 1 : 0;
+                         : occluded_coherent(s, o, d, max_distance[i], tally)) ? 1 : 0;
 }
 
 // Lane refill on one resident wave of CTAs (ray_route).  Warp w of W

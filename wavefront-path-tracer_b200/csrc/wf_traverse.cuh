@@ -592,7 +592,7 @@ WF_CALL TraceState trace_closest_binary(const DeviceScene& s, V3 o, V3 d, Tally&
 // isOccluded, device_traversal.cuh:1035-1113.  A pure disjunction of
 // independent tests, so an early return at the first hit gives the same bit.
 template <typename Tally>
-WF_CALL bool trace_any_binary(const DeviceScene& s, V3 o, V3 d, float t_max, Tally& tally) {
+WF_DEV bool occluded_coherent(const DeviceScene& s, V3 o, V3 d, float t_max, Tally& tally) {
     for (uint32_t i = 0; i < s.direct_sphere_count; ++i) {
         float t;
         tally.sphere();
@@ -621,6 +621,11 @@ WF_CALL bool trace_any_binary(const DeviceScene& s, V3 o, V3 d, float t_max, Tal
         }
     }
     return false;
+}
+
+template <typename Tally>
+WF_CALL bool trace_any_binary(const DeviceScene& s, V3 o, V3 d, float t_max, Tally& tally) {
+    return occluded_coherent(s, o, d, t_max, tally);
 }
 
 // Surface attributes of the winning primitive (the Hit fields the shading
