@@ -242,6 +242,30 @@ def test_touching_instances(check, offset, floor_yaw, box_yaw, stack):
     assert got["usable"] == 1 and got["hits"] > n // 3
 
 
+@pytest.mark.parametrize("rise", [0.0, 1e-7, 1e-6, 1e-5, 1e-4, 1e-3])
+def test_coincident_surfaces(check, rise):
+    """Every instance twice, the copies lifted by `rise`: most hits have
+    another at the same distance, which the BVH2s' order decides, or one close
+    behind, which it does not."""
+    for yaw in (0.0, 90.0):
+        s = touching_scene((0, 0, 0), box_yaw=yaw, stack=1)
+        copy = s.instances.copy()
+        copy["translation"][:, 1] += np.float32(rise)
+        s.instances = np.concatenate([s.instances, copy])
+        sp = np.zeros(40, abi.SPHERE_DTYPE)
+        sp["center"][:20] = np.random.default_rng(1).uniform(-8, 8, (20, 3))
+        sp["center"][20:] = sp["center"][:20] + np.float32([0, rise, 0])
+        sp["radius"], sp["accel"] = 0.7, abi.ACCEL_BVH
+        s.spheres = sp
+        rng = np.random.default_rng(8)
+        o = rng.uniform(-9, 9, (40_000, 3))
+        o[:, 1] = np.abs(o[:, 1]) ** np.where(np.arange(len(o)) % 2 == 0, 1.0, 0.1) - 0.9
+        got = check(s, make_rays(o, unit(rng.normal(0, 1, o.shape))))
+        # (lifted copies still share the planes of their sides)
+        share = got["redone"] / got["hits"]
+        assert share > 0.9 if rise == 0.0 else share < (0.5 if rise >= 1e-5 else 1.0)
+
+
 def test_touching_primitives_of_several_kinds(check):
     """An instance's faces on a static quad's plane, a direct list's and a
     sphere's, and a sphere on the floor instance."""

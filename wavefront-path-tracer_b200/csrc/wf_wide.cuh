@@ -20,11 +20,12 @@
 // culls by "entry < closestT", in its own visit order.  Its answer is the
 // closest candidate whatever the order when the entries of that candidate's
 // boxes (the TLAS leaf's, of the world ray, and the triangle's, of the local
-// one) lie before the distance of every other candidate.  So a ray whose
-// closest candidate has an entry, or another candidate, that is not clearly
-// (kNear) on its side is traced once more by trace_closest_binary.  Rays
-// through a shared edge of two triangles and rays between touching surfaces
-// are the usual cases.  Any-hit queries do not depend on the order.
+// one) lie before the distance of every other candidate.  The lane sees every
+// candidate up to kNear past the closest one and notes whether that holds for
+// certain (lane_near); a ray for which it may not is traced once more by
+// trace_closest_binary.  Rays through a shared edge of two triangles and hits
+// of coincident triangles are the usual cases.  Any-hit queries do not depend
+// on the order.
 //
 // Nodes are culled here only where no candidate below them can be the
 // closest.  A candidate's computed distance may lie before its own box, by
@@ -302,9 +303,10 @@ struct Lane {
 };
 enum : uint32_t {
     kStageTlas = 0, kStageBlas = 1, kStageDirect = 2, kStageDone = 3, kStageMask = 3,
-    kTie = 4,   // the visit order could decide: a candidate, or the closest one's entry, is near the closest one
+    kTie = 4,   // another candidate or the closest one's entry leaves the order a say
     kRedo = 8,  // the BVH2s must decide whatever comes
-    kHit = 16   // kAny: occluded
+    kHit = 16,  // kAny: occluded
+    kLate = 32  // the closest candidate's entry is past its distance
 };
 
 WF_DEV bool lane_done(const Lane& L) { return (L.state & kStageMask) == kStageDone; }
@@ -343,14 +345,19 @@ WF_DEV float box_limit(const Lane& L) {
 }
 
 // A closest-hit candidate at distance t <= L.t * kNear whose boxes start at
-// `entry`: returns whether it is the closest one so far, and notes whether
-// the order could matter.
+// `entry`: returns whether it is the closest one so far.  A new closest one
+// is certain when it and its entry lie before the former closest, and so
+// before every other, and the entry within the reach of what is seen; it stays
+// so until another turns up at its distance, or (kLate) maybe before its
+// entry.
 WF_DEV bool lane_near(Lane& L, float t, float entry) {
     if (t >= L.t) {
-        L.state |= kTie;
+        if ((L.state & kLate) || t == L.t) L.state |= kTie;
         return false;
     }
-    if (t * kNear >= L.t || entry > t * kNear) L.state |= kTie; else L.state &= ~kTie;
+    L.state &= ~(kTie | kLate);
+    if (entry > t) L.state |= kLate;
+    if (fmaxf(t, entry) >= L.t || entry > t * kNear) L.state |= kTie;
     L.t = t;
     return true;
 }
@@ -592,6 +599,13 @@ WF_DEV void lane_step(Lane& L, const DeviceScene& s, Sink& sink, Tally& tally) {
         lane_triangle<kAny>(L, s, sink, tally);
 }
 
+// Whether the finished ray's answer could depend on the visit order, or it
+// met something the wide test does not cover: trace_closest_binary /
+// trace_any_binary decide it.  The kernels that refill their lanes do that
+// after their loop: a call inside it would cost the loop some 20 registers
+// of spills.
+WF_DEV bool lane_doubt(const Lane& L) { return (L.state & (kTie | kRedo)) && !(L.state & kHit); }
+
 // Called once when the lane is done: the linear scan of a direct list
 // without a BVH.
 template <bool kAny, typename Tally, typename Sink>
@@ -609,13 +623,6 @@ WF_DEV void lane_finish(Lane& L, const DeviceScene& s, Sink& sink, Tally& tally)
         if (h.t < L.t) sink.hit(h.t, h.u, h.v, h.prim, h.inst);
     }
 }
-
-// Whether the finished ray's answer could depend on the visit order, or it
-// met something the wide test does not cover: trace_closest_binary /
-// trace_any_binary decide it.  The kernels that refill their lanes do that
-// after their loop: a call inside it would cost the loop some 20 registers
-// of spills.
-WF_DEV bool lane_doubt(const Lane& L) { return (L.state & (kTie | kRedo)) && !(L.state & kHit); }
 
 // ------------------------------------------------- one ray to its end
 // (Without a warp vote: keeping the lanes together by one at every step costs
