@@ -195,10 +195,13 @@ def test_stage_profile_times_the_kernels_of_the_graph(cuda, which, direct):
     dev.close()
 
 
-def test_scene_creation_does_not_wait_for_other_streams(cuda):
+@pytest.mark.parametrize("frequency", [4, 72])  # the builder's scratch under and over a megabyte
+def test_scene_creation_does_not_wait_for_other_streams(cuda, frequency):
     """A scene is made while another stream is busy for about a second."""
     torch = cuda
-    scene, _ = _scene("cornell", 64, 64)
+    scene = wfpt.Scene()
+    scene.add_mesh(scenes.geodesic_sphere(frequency, scene.add_material(wfpt.material(abi.MAT_DIFFUSE, (1, 1, 1)))))
+    scene.instances = scenes.instance(0)
     wfpt.DeviceScene(scene).close()  # loads the kernels
     torch.cuda.synchronize()
     busy = torch.cuda.Stream()

@@ -52,9 +52,21 @@ cudaError_t build_wide_bvh(DeviceScene& view, const std::vector<BvhRef>& roots, 
     // divides the size of those before it)
     static_assert(sizeof(BvhRef) % sizeof(uint32_t) == 0 && alignof(BvhRef) == sizeof(uint32_t), "packed after words");
     char* scratch = nullptr;
-    cudaError_t e = device_alloc_async(
-        reinterpret_cast<void**>(&scratch),
-        16 + capacity * (sizeof(uint2) + sizeof(uint32_t)) + root_count * sizeof(BvhRef), cudaStreamLegacy);
+    // A small scene keeps it: a stream-ordered allocation takes 0.8 ms, a large
+    // part of such a scene's creation, and cudaFree waits for other streams.
+    const size_t scratch_bytes =
+        16 + capacity * (sizeof(uint2) + sizeof(uint32_t)) + root_count * sizeof(BvhRef);
+    const bool keep_scratch = scratch_bytes <= (size_t(1) << 20);
+    cudaError_t e;
+    if (keep_scratch) {
+        e = device_alloc(reinterpret_cast<void**>(&scratch), scratch_bytes);
+        if (e == cudaSuccess) {
+            allocations.push_back(scratch);
+            bytes += scratch_bytes;
+        }
+    } else {
+        e = device_alloc_async(reinterpret_cast<void**>(&scratch), scratch_bytes, cudaStreamLegacy);
+    }
     uint32_t* counters = reinterpret_cast<uint32_t*>(scratch);
     uint2* bases = reinterpret_cast<uint2*>(scratch + 16);
     uint32_t* items = reinterpret_cast<uint32_t*>(bases + capacity);
@@ -95,7 +107,7 @@ cudaError_t build_wide_bvh(DeviceScene& view, const std::vector<BvhRef>& roots, 
         e = cudaGetLastError();
     }
     // the legacy stream alone: renders on other streams go on
-    if (scratch) cudaFreeAsync(scratch, cudaStreamLegacy);
+    if (scratch && !keep_scratch) cudaFreeAsync(scratch, cudaStreamLegacy);
     cudaError_t waited = cudaStreamSynchronize(cudaStreamLegacy);
     if (e == cudaSuccess) e = waited;
     if (e != cudaSuccess) {
