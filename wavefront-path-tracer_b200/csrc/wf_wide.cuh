@@ -1,7 +1,7 @@
 // Traversal of the compressed 8-wide BVHs (WideNode, wf_device.cuh): closest
 // hit and any hit as resumable per-lane state machines, used by every kernel
 // that traces rays but camera rays and frame guides, whose warps visit the
-// same BVH2 nodes together.
+// same BVH2 nodes together, and the ray batches of shallow scenes (ray_route).
 //
 // The node layout and the test of eight quantised child boxes against a
 // ray-order hit mask follow Ylitie, Karras and Laine, "Efficient Incoherent
@@ -338,7 +338,7 @@ struct NoSink {
 };
 
 // The distance that a box's own test compares with: the ray's length, or none
-// (a closest hit's order is for lane_near to judge).
+// (lane_near weighs a closest hit's).
 template <bool kAny>
 WF_DEV float box_limit(const Lane& L) {
     return kAny ? L.t : 1.0e30f;
